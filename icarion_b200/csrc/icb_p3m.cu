@@ -563,192 +563,71 @@ constexpr int kPPPoly = 10;     // degree of that polynomial
 // interpolated (relative error ~ (a r_c / kPPTable)^2 / 8 ~ 3e-8 at a r_c = 2).
 constexpr int kPPTable = 4096;
 
-// Field of one ion: CIC interpolation of the mesh field (+ particle-
-// particle correction).  Thread tt handles the ion in sorted slot tt (or
-// slots[tt]).
-template <bool REF_WEIGHTS, class GT, bool POLY>
-__device__ __forceinline__ void sc_gather_ion(uint32_t tt, const MeshGeom& g, const PPParams& pp,
+// Field of every ion in FP64 arithmetic (FP64 mesh) and of the reference's
+// periodic solver: CIC interpolation of the mesh field, plus, for P3M, the
+// particle-particle correction over the cells within the cutoff.  One thread
+// per ion in sorted order (blocks of consecutive ions share their partners in
+// L1); thread t takes sorted slot t, or slots[t] (this handle's ions among
+// peers' ions: n counts the own ions then).
+template <bool REF_WEIGHTS>
+__global__ void __launch_bounds__(256, 4) k_sc_gather(MeshGeom g, PPParams pp,
                             const double4* __restrict__ ps, const float4* __restrict__ pf,
                             const uint32_t* __restrict__ keys, const uint32_t* __restrict__ vals,
                             const uint32_t* __restrict__ start, uint32_t n, const uint32_t* __restrict__ slots,
-                            const GT* __restrict__ gx, const GT* __restrict__ gy, const GT* __restrict__ gz,
-                            double* __restrict__ ex, double* __restrict__ ey, double* __restrict__ ez,
-                            const double* tab, const float* tabf) {
-    // Every lane of a warp reaches the particle-particle loops (they use
-    // warp-wide ranges); lanes without an ion inside the mesh take part with
-    // empty ranges.
-    // thread t takes sorted slot t, or slots[t] (this handle's ions among
-    // peers' ions: n counts the own ions then)
-    const bool in_range = tt < n;
-    const uint32_t s = in_range ? (slots ? slots[tt] : tt) : 0u;
-    const uint32_t i = in_range ? vals[s] : 0u;
-    const uint32_t key = in_range ? keys[s] : g.ncell;
-    const bool act = key < g.ncell;
-    if (!REF_WEIGHTS && pp.on && pp.use_float && __all_sync(0xffffffffu, !act)) {
-        if (in_range) { ex[i] = 0.0; ey[i] = 0.0; ez[i] = 0.0; }
+                            const double* __restrict__ gx, const double* __restrict__ gy,
+                            const double* __restrict__ gz,
+                            double* __restrict__ ex, double* __restrict__ ey, double* __restrict__ ez) {
+    __shared__ double tab[REF_WEIGHTS ? 1 : kPPTable + 1];     // the long-range table
+    if (!REF_WEIGHTS && pp.on) {
+        for (int k = threadIdx.x; k <= kPPTable; k += blockDim.x) tab[k] = pp.table[k];
+        __syncthreads();
+    }
+    const uint32_t tt = blockIdx.x * blockDim.x + threadIdx.x;
+    if (tt >= n) return;
+    const uint32_t s = slots ? slots[tt] : tt;
+    const uint32_t i = vals[s];
+    const uint32_t key = keys[s];
+    if (key >= g.ncell) {
+        ex[i] = 0.0; ey[i] = 0.0; ez[i] = 0.0;
         return;
     }
-    if (!act && (REF_WEIGHTS || !pp.on || !pp.use_float)) {
-        if (in_range) { ex[i] = 0.0; ey[i] = 0.0; ez[i] = 0.0; }
-        return;
-    }
-    const uint32_t keyc = act ? key : 0u;
-    const int ck = static_cast<int>(keyc % g.n2);
-    const uint32_t t = keyc / g.n2;
+    const int ck = static_cast<int>(key % g.n2);
+    const uint32_t t = key / g.n2;
     const int cj = static_cast<int>(t % g.n1);
     const int ci = static_cast<int>(t / g.n1);
     double E[3] = {0.0, 0.0, 0.0};
-    const double4 pi4 = act ? ps[s] : make_double4(0.0, 0.0, 0.0, 0.0);
+    const double4 pi4 = ps[s];
     const double xi = pi4.x, yi = pi4.y, zi = pi4.z;
-    if (act) {
-        const double fx = (xi - g.lo0) * g.ih0 - ci;
-        const double fy = (yi - g.lo1) * g.ih1 - cj;
-        const double fz = (zi - g.lo2) * g.ih2 - ck;
-        const GT* grid[3] = {gx, gy, gz};
-        // corners in the reference's order w000, w100, w010, w110, w001, ... (x fastest)
-        for (int oz = 0; oz < 2; ++oz) {
-            for (int oy = 0; oy < 2; ++oy) {
-                for (int ox = 0; ox < 2; ++ox) {
-                    double w;
-                    if (REF_WEIGHTS) {
-                        w = static_cast<double>(cic_w<float>(ox, oy, oz, static_cast<float>(fx), static_cast<float>(fy),
-                                                             static_cast<float>(fz)));
-                    } else {
-                        w = cic_w<double>(ox, oy, oz, fx, fy, fz);
-                    }
-                    const size_t node = (static_cast<size_t>(ci + ox) * g.m1 + static_cast<size_t>(cj + oy)) * g.m2 +
-                                        static_cast<size_t>(ck + oz);
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) E[c] += w * static_cast<double>(grid[c][node]);
+    const double fx = (xi - g.lo0) * g.ih0 - ci;
+    const double fy = (yi - g.lo1) * g.ih1 - cj;
+    const double fz = (zi - g.lo2) * g.ih2 - ck;
+    const double* grid[3] = {gx, gy, gz};
+    // corners in the reference's order w000, w100, w010, w110, w001, ... (x fastest)
+    for (int oz = 0; oz < 2; ++oz) {
+        for (int oy = 0; oy < 2; ++oy) {
+            for (int ox = 0; ox < 2; ++ox) {
+                double w;
+                if (REF_WEIGHTS) {
+                    w = static_cast<double>(cic_w<float>(ox, oy, oz, static_cast<float>(fx), static_cast<float>(fy),
+                                                         static_cast<float>(fz)));
+                } else {
+                    w = cic_w<double>(ox, oy, oz, fx, fy, fz);
                 }
+                const size_t node = (static_cast<size_t>(ci + ox) * g.m1 + static_cast<size_t>(cj + oy)) * g.m2 +
+                                    static_cast<size_t>(ck + oz);
+#pragma unroll
+                for (int c = 0; c < 3; ++c) E[c] += w * grid[c][node];
             }
         }
-        if (REF_WEIGHTS) {
+    }
+    if (REF_WEIGHTS) {
 #pragma unroll
-            for (int c = 0; c < 3; ++c) E[c] = static_cast<double>(static_cast<float>(E[c]));
-        }
+        for (int c = 0; c < 3; ++c) E[c] = static_cast<double>(static_cast<float>(E[c]));
     }
     if (!REF_WEIGHTS && pp.on) {
         const int x0 = max(ci - pp.r0, 0), x1 = min(ci + pp.r0, g.n0 - 2);
         const int y0 = max(cj - pp.r1, 0), y1 = min(cj + pp.r1, g.n1 - 2);
         const int z0 = max(ck - pp.r2, 0), z1 = min(ck + pp.r2, g.n2 - 2);
-        if (pp.use_float) {
-            // float arithmetic on positions relative to the mesh origin,
-            // partners read as slot pairs (k_sc_permute) and evaluated two
-            // at a time on the packed FP32 pipe (sm_100 fma/add/mul .f32x2:
-            // one instruction for both).
-            // Each (cx, cy) column contributes the cells whose z interval
-            // reaches within r_c of the ion given the column's distance in x
-            // and y (lower bounds, padded for rounding).  The warp walks the
-            // union of its lanes' slot ranges together (one broadcast load
-            // per pair) only when that union is barely longer than the
-            // longest range; otherwise each lane walks its own range (the
-            // warp pays the longest, with nearby loads): over the sorted
-            // FT-ICR cloud this evaluates ~1.6 pairs per useful one where
-            // walking unions costs ~2.2.  Pairs outside a lane's range or
-            // outside (min_d, r_c) add exactly nothing (the ion itself is at
-            // distance 0 < min_d), so the sums equal a walk over every pair
-            // of the cells within reach.
-            const unsigned full = 0xffffffffu;
-            float fxi = 0.f, fyi = 0.f, fzi = 0.f;
-            if (act) {
-                const float* b = reinterpret_cast<const float*>(pf) + 8u * (s >> 1) + (s & 1u);
-                fxi = b[0]; fyi = b[2]; fzi = b[4];
-            }
-            const float h0 = static_cast<float>(1.0 / g.ih0), h1 = static_cast<float>(1.0 / g.ih1);
-            const float ih2 = static_cast<float>(g.ih2);
-            const float rcpad = pp.rc2f * 1.0001f;
-            const float zpad = 1e-4f * static_cast<float>(1.0 / g.ih2);
-            const float2 m1 = make_float2(-1.f, -1.f);
-            const float2 FX = make_float2(fxi, fxi), FY = make_float2(fyi, fyi), FZ = make_float2(fzi, fzi);
-            const float2 INV = make_float2(pp.inv_drf, pp.inv_drf), EPS = make_float2(pp.eps2f, pp.eps2f);
-            const float2 US = make_float2(pp.pu_s, pp.pu_s);
-            float2 E2x = make_float2(0.f, 0.f), E2y = E2x, E2z = E2x;
-            // partners 2k and 2k + 1 (ta, tb: inside the lane's range)
-            auto pair2 = [&](uint32_t k, bool ta, bool tb) {
-                const float4 xy = pf[2u * k], zq = pf[2u * k + 1u];
-                const float2 dX = __ffma2_rn(make_float2(xy.x, xy.y), m1, FX);
-                const float2 dY = __ffma2_rn(make_float2(xy.z, xy.w), m1, FY);
-                const float2 dZ = __ffma2_rn(make_float2(zq.x, zq.y), m1, FZ);
-                const float2 r2 = __ffma2_rn(dZ, dZ, __ffma2_rn(dY, dY, __fmul2_rn(dX, dX)));
-                const bool na = ta && r2.x < pp.rc2f && r2.x >= pp.min_d2f;
-                const bool nb = tb && r2.y < pp.rc2f && r2.y >= pp.min_d2f;
-                const float2 ri = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
-                const float2 re = __fadd2_rn(r2, EPS);
-                const float2 rc = make_float2(__fdividef(1.f, re.x), __fdividef(1.f, re.y));
-                // 1 / ((r^2 + eps^2) r) - L(r) / r^3
-                float2 gsr;
-                if (POLY) {
-                    const float2 u = __ffma2_rn(r2, US, m1);
-                    float2 nP = make_float2(pp.pc[kPPPoly], pp.pc[kPPPoly]);
-#pragma unroll
-                    for (int c = kPPPoly - 1; c >= 0; --c) nP = __ffma2_rn(nP, u, make_float2(pp.pc[c], pp.pc[c]));
-                    gsr = __ffma2_rn(ri, rc, nP);
-                } else {
-                    const float2 uu = __fmul2_rn(__fmul2_rn(r2, ri), INV);
-                    const int ka = max(min(static_cast<int>(uu.x), kPPTable - 1), 0);
-                    const int kb = max(min(static_cast<int>(uu.y), kPPTable - 1), 0);
-                    const float2 fr = __ffma2_rn(make_float2(static_cast<float>(ka), static_cast<float>(kb)), m1, uu);
-                    const float2 t0 = make_float2(tabf[ka], tabf[kb]), t1 = make_float2(tabf[ka + 1], tabf[kb + 1]);
-                    const float2 L = __ffma2_rn(fr, __ffma2_rn(t0, m1, t1), t0);
-                    const float2 nri2 = __fmul2_rn(ri, __fmul2_rn(ri, m1));           // -1 / r^2
-                    gsr = __fmul2_rn(__ffma2_rn(L, nri2, rc), ri);
-                }
-                // kc q_j times that (zq.zw = kc q)
-                const float2 f = __fmul2_rn(gsr, make_float2(zq.z, zq.w));
-                const float2 sc = make_float2(na ? f.x : 0.f, nb ? f.y : 0.f);
-                E2x = __ffma2_rn(dX, sc, E2x);
-                E2y = __ffma2_rn(dY, sc, E2y);
-                E2z = __ffma2_rn(dZ, sc, E2z);
-            };
-            // slot range [sa, sb) of column (cx, cy) for this ion (dxa: its
-            // distance to the column's x slab)
-            auto column = [&](int cx, float dxa, int cy, uint32_t& sa, uint32_t& sb) {
-                sa = 0u;
-                sb = 0u;
-                const float dya = fmaxf(0.f, fmaxf(static_cast<float>(cy) * h1 - fyi,
-                                                   fyi - static_cast<float>(cy + 1) * h1));
-                const float rem = rcpad - dxa * dxa - dya * dya;
-                if (rem > 0.f) {
-                    const float dzm = sqrtf(rem) + zpad;
-                    const int za = max(z0, static_cast<int>(floorf((fzi - dzm) * ih2)));
-                    const int zb = min(z1, static_cast<int>(floorf((fzi + dzm) * ih2)));
-                    if (za <= zb) {
-                        const uint32_t row = (static_cast<uint32_t>(cx) * g.n1 + static_cast<uint32_t>(cy)) * g.n2;
-                        sa = start[row + static_cast<uint32_t>(za)];
-                        sb = start[row + static_cast<uint32_t>(zb) + 1u];
-                    }
-                }
-            };
-            auto slab = [&](int cx) {
-                return fmaxf(0.f, fmaxf(static_cast<float>(cx) * h0 - fxi, fxi - static_cast<float>(cx + 1) * h0));
-            };
-            const int wx0 = __reduce_min_sync(full, act ? x0 : INT_MAX);
-            const int wx1 = __reduce_max_sync(full, act ? x1 : INT_MIN);
-            const int wy0 = __reduce_min_sync(full, act ? y0 : INT_MAX);
-            const int wy1 = __reduce_max_sync(full, act ? y1 : INT_MIN);
-            for (int cx = wx0; cx <= wx1; ++cx) {
-                const float dxa = slab(cx);
-                for (int cy = wy0; cy <= wy1; ++cy) {
-                    uint32_t sa = 0u, sb = 0u;
-                    if (act && cx >= x0 && cx <= x1 && cy >= y0 && cy <= y1) column(cx, dxa, cy, sa, sb);
-                    const bool has = sb > sa;
-                    const uint32_t usa = __reduce_min_sync(full, has ? sa : 0xffffffffu);
-                    const uint32_t usb = __reduce_max_sync(full, has ? sb : 0u);
-                    if (usb <= usa) continue;                  // no lane has pairs in this column
-                    const uint32_t len = __reduce_max_sync(full, sb - sa);
-                    if (usb - usa <= len + (len >> 3) + 2u) {
-                        for (uint32_t k = usa >> 1; 2u * k < usb; ++k)
-                            pair2(k, 2u * k >= sa && 2u * k < sb, 2u * k + 1u >= sa && 2u * k + 1u < sb);
-                    } else {
-                        for (uint32_t k = sa >> 1; 2u * k < sb; ++k) pair2(k, 2u * k >= sa, 2u * k + 1u < sb);
-                    }
-                }
-            }
-            const float Ef[3] = {E2x.x + E2x.y, E2y.x + E2y.y, E2z.x + E2z.y};
-#pragma unroll
-            for (int c = 0; c < 3; ++c) E[c] += static_cast<double>(Ef[c]);
-        } else if (!POLY) {
         const float4 own = pf[s];
         for (int cx = x0; cx <= x1; ++cx) {
             for (int cy = y0; cy <= y1; ++cy) {
@@ -776,40 +655,180 @@ __device__ __forceinline__ void sc_gather_ion(uint32_t tt, const MeshGeom& g, co
                 }
             }
         }
-        }
-    }
-    if (!act) {
-        if (in_range) { ex[i] = 0.0; ey[i] = 0.0; ez[i] = 0.0; }
-        return;
     }
     ex[i] = E[0]; ey[i] = E[1]; ez[i] = E[2];
 }
 
-// Field of every ion, one thread per ion in sorted order (blocks of
-// consecutive ions share their partners in L1).  The polynomial form runs
-// blocks of 128: finer blocks leave fewer warps waiting for their block's
-// slowest one (the cloud's dense middle costs many times its edges).
-template <bool REF_WEIGHTS, class GT, bool POLY = false>
-__global__ void __launch_bounds__(POLY ? 128 : 256, POLY ? 8 : 4) k_sc_gather(MeshGeom g, PPParams pp,
+// 1/sqrt(x) and 1/x of normal floats by the hardware approximations (the
+// values of rsqrtf and __fdividef(1, x), without their denormal handling:
+// a denormal squared distance lies below min_d2 and is masked).
+__device__ __forceinline__ float rsqrt_hw(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float rcp_hw(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+// Field of every ion of the isolated solver's single-precision form: CIC
+// interpolation of the float mesh field and the particle-particle correction
+// in float arithmetic on positions relative to the mesh origin.
+//
+// Four lanes per ion, eight consecutive sorted ions per warp.  Partners are
+// read as slot pairs (k_sc_permute) and evaluated two at a time on the packed
+// FP32 pipe (fma/add/mul .f32x2).  Each (x, y) neighbour column contributes
+// the z cells that reach within r_c of the ion given the column's distance
+// (lower bounds, padded for rounding): the ion's four lanes set up four
+// columns at once, then walk each column's slot range together, lane j
+// taking every fourth slot pair.  Pairs outside the range or outside
+// (min_d, r_c) add exactly nothing (the ion itself is at distance 0).
+constexpr int kGatherBlock = 128;
+constexpr int kGatherLanes = 4;
+
+template <bool POLY>
+__global__ void __launch_bounds__(kGatherBlock, 8) k_sc_gather_f32(MeshGeom g, PPParams pp,
                             const double4* __restrict__ ps, const float4* __restrict__ pf,
                             const uint32_t* __restrict__ keys, const uint32_t* __restrict__ vals,
                             const uint32_t* __restrict__ start, uint32_t n, const uint32_t* __restrict__ slots,
-                            const GT* __restrict__ gx, const GT* __restrict__ gy, const GT* __restrict__ gz,
+                            const float* __restrict__ gx, const float* __restrict__ gy, const float* __restrict__ gz,
                             double* __restrict__ ex, double* __restrict__ ey, double* __restrict__ ez) {
-    // the long-range table (the polynomial form has none; it runs with the
-    // float loop only)
-    __shared__ double tab[(REF_WEIGHTS || POLY) ? 1 : kPPTable + 1];
-    float* tabf = reinterpret_cast<float*>(tab);
-    if (!REF_WEIGHTS && !POLY && pp.on) {
-        if (pp.use_float) {
-            for (int k = threadIdx.x; k <= kPPTable; k += blockDim.x) tabf[k] = static_cast<float>(pp.table[k]);
-        } else {
-            for (int k = threadIdx.x; k <= kPPTable; k += blockDim.x) tab[k] = pp.table[k];
-        }
+    __shared__ float tabf[POLY ? 1 : kPPTable + 1];            // the long-range table
+    if (!POLY) {
+        for (int k = threadIdx.x; k <= kPPTable; k += blockDim.x) tabf[k] = static_cast<float>(pp.table[k]);
         __syncthreads();
     }
-    sc_gather_ion<REF_WEIGHTS, GT, POLY>(blockIdx.x * blockDim.x + threadIdx.x, g, pp, ps, pf, keys, vals, start, n,
-                                         slots, gx, gy, gz, ex, ey, ez, tab, tabf);
+    const unsigned full = 0xffffffffu;
+    const uint32_t jl = threadIdx.x & (kGatherLanes - 1);
+    const uint32_t tt = (blockIdx.x * blockDim.x + threadIdx.x) / kGatherLanes;
+    // sorted slot tt, or slots[tt] (this handle's ions among peers' ions: n
+    // counts the own ions then)
+    const bool in_range = tt < n;
+    const uint32_t s = in_range ? (slots ? slots[tt] : tt) : 0u;
+    const uint32_t key = in_range ? keys[s] : g.ncell;
+    const bool act = key < g.ncell;
+    double E[3] = {0.0, 0.0, 0.0};
+    if (__any_sync(full, act)) {
+        const uint32_t keyc = act ? key : 0u;
+        const int ck = static_cast<int>(keyc % g.n2);
+        const uint32_t t = keyc / g.n2;
+        const int cj = static_cast<int>(t % g.n1);
+        const int ci = static_cast<int>(t / g.n1);
+        float fxi = 0.f, fyi = 0.f, fzi = 0.f;
+        if (act) {
+            // lane j: the two z corners of the cell's (x, y) edge j
+            const double4 pi4 = ps[s];
+            const double fx = (pi4.x - g.lo0) * g.ih0 - ci;
+            const double fy = (pi4.y - g.lo1) * g.ih1 - cj;
+            const double fz = (pi4.z - g.lo2) * g.ih2 - ck;
+            const int ox = static_cast<int>(jl >> 1), oy = static_cast<int>(jl & 1u);
+            const size_t node = (static_cast<size_t>(ci + ox) * g.m1 + static_cast<size_t>(cj + oy)) * g.m2 +
+                                static_cast<size_t>(ck);
+            const double w0 = cic_w<double>(ox, oy, 0, fx, fy, fz), w1 = cic_w<double>(ox, oy, 1, fx, fy, fz);
+            E[0] = w0 * static_cast<double>(gx[node]) + w1 * static_cast<double>(gx[node + 1]);
+            E[1] = w0 * static_cast<double>(gy[node]) + w1 * static_cast<double>(gy[node + 1]);
+            E[2] = w0 * static_cast<double>(gz[node]) + w1 * static_cast<double>(gz[node + 1]);
+            const float* b = reinterpret_cast<const float*>(pf) + 8u * (s >> 1) + (s & 1u);
+            fxi = b[0]; fyi = b[2]; fzi = b[4];
+        }
+        const int z0 = max(ck - pp.r2, 0), z1 = min(ck + pp.r2, g.n2 - 2);
+        const float h0 = static_cast<float>(1.0 / g.ih0), h1 = static_cast<float>(1.0 / g.ih1);
+        const float ih2 = static_cast<float>(g.ih2);
+        const float rcpad = pp.rc2f * 1.0001f;
+        const float zpad = 1e-4f * static_cast<float>(1.0 / g.ih2);
+        const float2 m1 = make_float2(-1.f, -1.f);
+        const float2 FX = make_float2(fxi, fxi), FY = make_float2(fyi, fyi), FZ = make_float2(fzi, fzi);
+        const float2 INV = make_float2(pp.inv_drf, pp.inv_drf), EPS = make_float2(pp.eps2f, pp.eps2f);
+        const float2 US = make_float2(pp.pu_s, pp.pu_s);
+        float2 E2x = make_float2(0.f, 0.f), E2y = E2x, E2z = E2x;
+        const int ncol = (2 * pp.r0 + 1) * (2 * pp.r1 + 1);
+        int dcx = -pp.r0, dcy = -pp.r1 + static_cast<int>(jl);    // this lane's next column
+        for (int c0 = 0; c0 < ncol; c0 += kGatherLanes) {
+            while (dcy > pp.r1) { dcy -= 2 * pp.r1 + 1; ++dcx; }
+            const int cx = ci + dcx, cy = cj + dcy;
+            dcy += kGatherLanes;
+            uint32_t sa = 0u, sb = 0u;
+            if (act && c0 + static_cast<int>(jl) < ncol && cx >= 0 && cx <= g.n0 - 2 && cy >= 0 && cy <= g.n1 - 2) {
+                const float dxa = fmaxf(0.f, fmaxf(static_cast<float>(cx) * h0 - fxi,
+                                                   fxi - static_cast<float>(cx + 1) * h0));
+                const float dya = fmaxf(0.f, fmaxf(static_cast<float>(cy) * h1 - fyi,
+                                                   fyi - static_cast<float>(cy + 1) * h1));
+                const float rem = rcpad - dxa * dxa - dya * dya;
+                if (rem > 0.f) {
+                    const float dzm = sqrtf(rem) + zpad;
+                    const int za = max(z0, static_cast<int>(floorf((fzi - dzm) * ih2)));
+                    const int zb = min(z1, static_cast<int>(floorf((fzi + dzm) * ih2)));
+                    if (za <= zb) {
+                        const uint32_t row = (static_cast<uint32_t>(cx) * g.n1 + static_cast<uint32_t>(cy)) * g.n2;
+                        sa = start[row + static_cast<uint32_t>(za)];
+                        sb = start[row + static_cast<uint32_t>(zb) + 1u];
+                    }
+                }
+            }
+#pragma unroll 1
+            for (int q = 0; q < kGatherLanes; ++q) {
+                const uint32_t a = __shfl_sync(full, sa, q, kGatherLanes), e = __shfl_sync(full, sb, q, kGatherLanes);
+                for (uint32_t k2 = (a & ~1u) + 2u * jl; k2 < e; k2 += 2u * kGatherLanes) {
+                    // partners k2 and k2 + 1
+                    const float4 xy = pf[k2], zq = pf[k2 + 1u];
+                    const float2 dX = __ffma2_rn(make_float2(xy.x, xy.y), m1, FX);
+                    const float2 dY = __ffma2_rn(make_float2(xy.z, xy.w), m1, FY);
+                    const float2 dZ = __ffma2_rn(make_float2(zq.x, zq.y), m1, FZ);
+                    const float2 r2 = __ffma2_rn(dZ, dZ, __ffma2_rn(dY, dY, __fmul2_rn(dX, dX)));
+                    const bool na = k2 >= a && r2.x < pp.rc2f && r2.x >= pp.min_d2f;
+                    const bool nb = k2 + 1u < e && r2.y < pp.rc2f && r2.y >= pp.min_d2f;
+                    const float2 ri = make_float2(rsqrt_hw(r2.x), rsqrt_hw(r2.y));
+                    const float2 re = __fadd2_rn(r2, EPS);
+                    const float2 rc = make_float2(rcp_hw(re.x), rcp_hw(re.y));
+                    // 1 / ((r^2 + eps^2) r) - L(r) / r^3
+                    float2 gsr;
+                    if (POLY) {
+                        const float2 u = __ffma2_rn(r2, US, m1);
+                        float2 nP = make_float2(pp.pc[kPPPoly], pp.pc[kPPPoly]);
+#pragma unroll
+                        for (int c = kPPPoly - 1; c >= 0; --c)
+                            nP = __ffma2_rn(nP, u, make_float2(pp.pc[c], pp.pc[c]));
+                        gsr = __ffma2_rn(ri, rc, nP);
+                    } else {
+                        const float2 uu = __fmul2_rn(__fmul2_rn(r2, ri), INV);
+                        const int ka = max(min(static_cast<int>(uu.x), kPPTable - 1), 0);
+                        const int kb = max(min(static_cast<int>(uu.y), kPPTable - 1), 0);
+                        const float2 fr = __ffma2_rn(make_float2(static_cast<float>(ka), static_cast<float>(kb)), m1, uu);
+                        const float2 t0 = make_float2(tabf[ka], tabf[kb]), t1 = make_float2(tabf[ka + 1], tabf[kb + 1]);
+                        const float2 L = __ffma2_rn(fr, __ffma2_rn(t0, m1, t1), t0);
+                        const float2 nri2 = __fmul2_rn(ri, __fmul2_rn(ri, m1));           // -1 / r^2
+                        gsr = __fmul2_rn(__ffma2_rn(L, nri2, rc), ri);
+                    }
+                    // kc q_j times that (zq.zw = kc q)
+                    const float2 f = __fmul2_rn(gsr, make_float2(zq.z, zq.w));
+                    const float2 sc = make_float2(na ? f.x : 0.f, nb ? f.y : 0.f);
+                    E2x = __ffma2_rn(dX, sc, E2x);
+                    E2y = __ffma2_rn(dY, sc, E2y);
+                    E2z = __ffma2_rn(dZ, sc, E2z);
+                }
+            }
+        }
+        float Ef[3] = {E2x.x + E2x.y, E2y.x + E2y.y, E2z.x + E2z.y};
+#pragma unroll
+        for (int o = 1; o < kGatherLanes; o <<= 1) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                Ef[c] += __shfl_xor_sync(full, Ef[c], o);
+                E[c] += __shfl_xor_sync(full, E[c], o);
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < 3; ++c) E[c] += static_cast<double>(Ef[c]);
+    }
+    // lane c writes component c
+    if (in_range) {
+        const uint32_t i = vals[s];
+        if (jl == 0u) ex[i] = act ? E[0] : 0.0;
+        else if (jl == 1u) ey[i] = act ? E[1] : 0.0;
+        else if (jl == 2u) ez[i] = act ? E[2] : 0.0;
+    }
 }
 
 // L(r) / (a r)^3 as a function of x = (a r)^2: (erf(t) - 2t e^(-x) / sqrt(pi)) / t^3
@@ -1303,9 +1322,8 @@ int sc_solve(SpaceChargeSolver* S, const double* x, const double* y, const doubl
             SC_FFT(cufftExecC2R(S->inv2, S->tmp_hat_f + c * cs, S->egrid_f + c * ms));
         }
         }
-        auto gather = S->pp.poly ? k_sc_gather<false, float, true> : k_sc_gather<false, float, false>;
-        const int gb = S->pp.poly ? 128 : 256;
-        gather<<<blocks_for(n_gather, gb), gb, 0, s>>>(
+        auto gather = S->pp.poly ? k_sc_gather_f32<true> : k_sc_gather_f32<false>;
+        gather<<<blocks_for(static_cast<size_t>(n_gather) * kGatherLanes, kGatherBlock), kGatherBlock, 0, s>>>(
             g, S->pp, S->ps, S->pf, S->keys_sorted, S->vals_sorted, S->start, n_gather, slots, S->egrid_f,
             S->egrid_f + ms, S->egrid_f + 2 * ms, S->esc[0], S->esc[1], S->esc[2]);
         SC_CUDA(cudaGetLastError());
@@ -1318,7 +1336,7 @@ int sc_solve(SpaceChargeSolver* S, const double* x, const double* y, const doubl
                                                                     S->tmp_hat, S->cplx_size());
         SC_CUDA(cudaGetLastError());
         SC_FFT(cufftExecZ2D(S->inv3, S->tmp_hat, S->egrid[0]));
-        k_sc_gather<false, double><<<blocks_for(n_gather, 256), 256, 0, s>>>(
+        k_sc_gather<false><<<blocks_for(n_gather, 256), 256, 0, s>>>(
             g, S->pp, S->ps, S->pf, S->keys_sorted, S->vals_sorted, S->start, n_gather, slots, S->egrid[0],
             S->egrid[1], S->egrid[2], S->esc[0], S->esc[1], S->esc[2]);
         SC_CUDA(cudaGetLastError());
@@ -1334,7 +1352,7 @@ int sc_solve(SpaceChargeSolver* S, const double* x, const double* y, const doubl
         k_sc_efield_ref<<<blocks_for(S->real_size(), 256), 256, 0, s>>>(g, S->h[0], S->h[1], S->h[2], scale, S->rho,
                                                                          S->egrid[0], S->egrid[1], S->egrid[2]);
         SC_CUDA(cudaGetLastError());
-        k_sc_gather<true, double><<<blocks_for(n_gather, 256), 256, 0, s>>>(
+        k_sc_gather<true><<<blocks_for(n_gather, 256), 256, 0, s>>>(
             g, S->pp, S->ps, S->pf, S->keys_sorted, S->vals_sorted, S->start, n_gather, slots, S->egrid[0],
             S->egrid[1], S->egrid[2], S->esc[0], S->esc[1], S->esc[2]);
         SC_CUDA(cudaGetLastError());
