@@ -102,18 +102,6 @@ __global__ void k_clock_init(R* S, R* U, uint32_t* nxt, uint32_t* start, uint64_
     }
 }
 
-// Device engine clock: step += K and t_e += dt_e, K times (accumulated like
-// the engine's per-step t += dt, SimulationEngineLifecycle.cpp:162).
-__global__ void k_clock_advance(unsigned long long* step, double* t, const double* dt, int n_ens, uint32_t K) {
-    const int e = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
-    if (e == 0) *step += K;
-    if (e >= n_ens) return;
-    double te = t[e];
-    const double d = dt[e];
-    for (uint32_t k = 0; k < K; ++k) te = te + d;
-    t[e] = te;
-}
-
 // Upload conversion: staged doubles -> working precision.
 __global__ void k_to_float(const double* __restrict__ src, float* __restrict__ dst, uint64_t n) {
     const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -797,6 +785,19 @@ uint32_t tf_stride(const icb_handle* h) {
     return static_cast<uint32_t>(kTfRowScalars * (h->cfg.integrator == ICB_INTEGRATOR_RK4 ? 2 : 1));
 }
 
+// Whether a launch of K steps reads a per-step table: a time-dependent field
+// always does; constant-voltage RF and AC ensembles when the launch is long
+// enough to pay for the table's own launch (about 5 us; the cosines cost a
+// lane 0.3 us each and step when the chip is not full, more when it is).
+constexpr uint32_t kRfTabSteps = 16;
+bool rf_tab(const icb_handle* h, uint32_t K) {
+    if (K < kRfTabSteps) return false;
+    for (const EnsConst& C : h->ens_const)
+        if (!C.tf && (C.rf || C.ac)) return true;
+    return false;
+}
+bool needs_tab(const icb_handle* h, uint32_t K) { return h->any_tf || rf_tab(h, K); }
+
 // Room for the per-step field tables of launches of up to K steps (all
 // ensembles, plus the time sequences); allocates outside stream capture only.
 int ensure_tf_tab(icb_handle* h, uint32_t K, cudaStream_t st) {
@@ -823,7 +824,7 @@ int ensure_tf_tab(icb_handle* h, uint32_t K, cudaStream_t st) {
 // ensembles with a time-dependent field, built on `st` before the step
 // kernels read them (stage 0 at t_k; RK4 adds the half step).
 int enqueue_tf_tables(icb_handle* h, uint32_t K, cudaStream_t st) {
-    if (!h->any_tf) return ICB_OK;
+    if (!needs_tab(h, K)) return ICB_OK;
     if (int r = ensure_tf_tab(h, K, st)) return r;
     const uint32_t stride = tf_stride(h);
     const int n_ens = static_cast<int>(h->ens.size());
@@ -837,6 +838,7 @@ int enqueue_tf_tables(icb_handle* h, uint32_t K, cudaStream_t st) {
         p.n_steps = K;
         p.ens_base = static_cast<uint32_t>(e0);
         p.n_ens = static_cast<uint32_t>(ne);
+        p.tab_fused = h->fp64() ? 0u : 1u;
         for (int e = 0; e < ne; ++e) p.ens[e] = h->ens_const[static_cast<size_t>(e0 + e)];
         const cudaError_t te = launch_tf_table(p, h->tf_tab.p, tseq, stride, st);
         ++h->launches;
@@ -923,9 +925,10 @@ int launch_step(icb_handle* h, uint32_t K, int do_push, int do_collide, int do_f
             p.ens[e] = h->ens_const[static_cast<size_t>(e0 + e)];
             if (p.ens[e].flow) p.flows = 1u;
         }
-        if (h->any_tf) {
+        if (needs_tab(h, K)) {
             p.tf_tab = h->tf_tab.p;
             p.tf_stride = tf_stride(h);
+            p.rf_tab = rf_tab(h, K) ? 1u : 0u;
         }
         if (h->cfg.collision_test == ICB_TEST_PER_STEP) {
             // the per-step kernel: fused steps only, none of the per-launch extras
@@ -1015,8 +1018,7 @@ int enqueue_advance(icb_handle* h, uint64_t n_steps, size_t n_timed) {
         if (j < n_timed) ICB_CUDA(cudaEventRecord(h->kev[2 * j], s));
         if (int r = launch_step(h, K, 1, 1, 1)) return r;
         if (j < n_timed) ICB_CUDA(cudaEventRecord(h->kev[2 * j + 1], s));
-        k_clock_advance<<<(ne + 127) / 128, 128, 0, s>>>(h->step_dev.p, h->t_dev.p, h->dt_dev.p, ne, K);
-        ICB_CUDA(cudaGetLastError());
+        ICB_CUDA(launch_clock_advance(h->step_dev.p, h->t_dev.p, h->dt_dev.p, ne, K, s));
         ++h->launches;
         left -= K;
         ++j;
@@ -1498,8 +1500,9 @@ int icb_advance(icb_handle* h, uint64_t n_steps, icb_run_stats* stats) {
             // Captured on the handle's own non-blocking stream (capture is
             // not allowed on the legacy default stream); replayed on h->stream.
             cudaGraph_t g = nullptr;
-            if (h->any_tf) {
-                if (int r = ensure_tf_tab(h, static_cast<uint32_t>(std::min<uint64_t>(n_steps, h->K)), s)) return r;
+            const uint32_t Kg = h->sc ? 1u : static_cast<uint32_t>(std::min<uint64_t>(n_steps, h->K));
+            if (needs_tab(h, Kg)) {
+                if (int r = ensure_tf_tab(h, Kg, s)) return r;
             }
             ICB_CUDA(cudaStreamBeginCapture(h->own_stream, cudaStreamCaptureModeThreadLocal));
             h->stream = h->own_stream;
@@ -1986,9 +1989,7 @@ int icb_advance_host(icb_handle* h, uint64_t n_steps, int n_chunks, double* x, d
     ICB_CUDA(cudaEventRecord(h->hev[2 * n_chunks], bs));
     ICB_CUDA(cudaStreamWaitEvent(s, h->hev[2 * n_chunks], 0));
     const int ne = static_cast<int>(h->ens.size());
-    k_clock_advance<<<(ne + 127) / 128, 128, 0, s>>>(h->step_dev.p, h->t_dev.p, h->dt_dev.p, ne,
-                                                      static_cast<uint32_t>(n_steps));
-    ICB_CUDA(cudaGetLastError());
+    ICB_CUDA(launch_clock_advance(h->step_dev.p, h->t_dev.p, h->dt_dev.p, ne, static_cast<uint32_t>(n_steps), s));
     ++h->launches;
     ICB_CUDA(cudaEventRecord(h->ev1, s));
     if (stats) return read_stats(h, stats, n_steps, 0);
@@ -2013,8 +2014,7 @@ static int single_part(icb_handle* h, int push, int collide, int finalize, icb_r
     if (int r = launch_step(h, 1, push, collide, finalize)) return r;
     if (finalize) {
         const int ne = static_cast<int>(h->ens.size());
-        k_clock_advance<<<(ne + 127) / 128, 128, 0, s>>>(h->step_dev.p, h->t_dev.p, h->dt_dev.p, ne, 1);
-        ICB_CUDA(cudaGetLastError());
+        ICB_CUDA(launch_clock_advance(h->step_dev.p, h->t_dev.p, h->dt_dev.p, ne, 1u, s));
         ++h->launches;
     }
     ICB_CUDA(cudaEventRecord(h->ev1, s));

@@ -186,6 +186,8 @@ struct StepParams {
     // k = 0..n_steps of tf_stride doubles per chunk ensemble; nullable
     const double* tf_tab;
     uint32_t tf_stride;
+    uint32_t rf_tab;                   // tf_tab has rows for the constant-voltage RF / AC ensembles too
+    uint32_t tab_fused;                // k_tf_table: a phase sum w t + phase as one fused operation
     // EHSS molecule geometry: atoms (x, y, z, radius) of ensemble e in
     // [ehss_off[e], ehss_off[e+1]), gas (contact) radius per ensemble
     const double4* ehss_atoms;

@@ -13,7 +13,14 @@ cudaError_t launch_step_fp64(int integ, int coll, int field, bool mag, const Ste
 }
 
 cudaError_t launch_tf_table(const StepParams& p, double* tab, double* tseq, uint32_t stride, cudaStream_t s) {
-    k_tf_table<<<p.n_ens, 128, 0, s>>>(p, tab, tseq, stride);
+    k_tf_table<<<p.n_ens, 256, 0, s>>>(p, tab, tseq, stride);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_clock_advance(unsigned long long* step, double* t, const double* dt, int n_ens, uint32_t K,
+                                 cudaStream_t s) {
+    // a launch of few steps needs no more than a warp
+    k_clock_advance<<<n_ens, K >= 64u ? 256 : 32, 0, s>>>(step, t, dt, K);
     return cudaGetLastError();
 }
 }  // namespace icb

@@ -88,6 +88,34 @@ __device__ __forceinline__ float m_one_minus_exp(float x) {
     }
     return 1.0f - __expf(-x);
 }
+// a / b for a divisor that stays the same for a whole launch, y = RN(1 / b),
+// b > 0 in [2^-300, 2^300] (checked where y is formed: y = 0 otherwise): the
+// correctly rounded quotient by Markstein's correction (IBM J. Res. Dev. 34,
+// 1990: with y the rounded reciprocal and q within an ulp of a / b,
+// RN(q + RN(a - b q) y) is RN(a / b)); the first correction brings q = a y
+// within an ulp.  Five dependent operations instead of the general
+// division's reciprocal iteration and range handling.  Dividends outside
+// [2^-623, 2^577] (and NaN) take the general division, zero keeps a y.
+static __device__ __noinline__ double div_general(double a, double b) { return a / b; }
+__device__ __forceinline__ double div_by(double a, double b, double y) {
+    const double q = a * y;
+    const uint32_t ea = (static_cast<uint32_t>(__double2hiint(a)) >> 20) & 0x7ffu;
+    if (ea - 400u >= 1200u || y == 0.0) return (a == 0.0 && y != 0.0) ? q : div_general(a, b);
+    const double q1 = fma(fma(-b, q, a), y, q);
+    return fma(fma(-b, q1, a), y, q1);
+}
+__device__ __forceinline__ double div_reciprocal(double b) {
+    const uint32_t eb = (static_cast<uint32_t>(__double2hiint(b)) >> 20);      // b > 0: sign bit clear
+    return eb - 723u < 601u ? 1.0 / b : 0.0;
+}
+// Float forms: one hardware reciprocal per launch instead of one per step
+// (the values of -prec-div=false division, a times that reciprocal).
+__device__ __forceinline__ float div_by(float a, float, float y) { return a * y; }
+__device__ __forceinline__ float div_reciprocal(float b) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
+    return y;
+}
 __device__ __forceinline__ double m_fmax(double a, double b) { return fmax(a, b); }
 __device__ __forceinline__ float m_fmax(float a, float b) { return fmaxf(a, b); }
 __device__ __forceinline__ double m_fmin(double a, double b) { return fmin(a, b); }
@@ -133,7 +161,8 @@ struct PosD {
     __device__ Snap snap_z() const { return z; }
     __device__ double z_of(Snap s) const { return s; }
     __device__ void fold() {}
-    template <class R> __device__ R rel(int a, double c) const {
+    __device__ void refer(const double[3]) {}
+    template <class R> __device__ R at(int a, double c) const {
         const double v = (a == 0) ? x : (a == 1) ? y : z;
         return static_cast<R>(v - c);
     }
@@ -148,10 +177,23 @@ struct PosD {
 // offset (one FFMA per axis, no conversion); every lane folds the offset
 // into the anchor at each warp vote (every steps_per_vote steps), so the
 // offset stays below ~1 um and its rounding below ~1e-13 m per step.
+//
+// rx, ry, rz: the anchor's float distance from the field's reference point,
+// taken when the anchor moves (refer) instead of at every field evaluation
+// (three double subtractions and conversions a step: the 262,144-ion TIMS
+// pass of 500 steps 1843 -> 1704 us; kernels without a position-dependent
+// field never form it).
 struct PosA {
     using Snap = float;
     double ax, ay, az;
     float dx, dy, dz;
+    float rx, ry, rz;
+    __device__ void refer(const double c[3]) {
+        rx = static_cast<float>(ax - c[0]); ry = static_cast<float>(ay - c[1]); rz = static_cast<float>(az - c[2]);
+    }
+    template <class R> __device__ R at(int a, double) const {
+        return static_cast<R>(a == 0 ? rx + dx : a == 1 ? ry + dy : rz + dz);
+    }
     __device__ void load(const StepParams& p, uint64_t i) {
         ax = p.x[i]; ay = p.y[i]; az = p.z[i];
         dx = dy = dz = 0.0f;
@@ -165,11 +207,6 @@ struct PosA {
     __device__ void fold() {
         ax += static_cast<double>(dx); ay += static_cast<double>(dy); az += static_cast<double>(dz);
         dx = dy = dz = 0.0f;
-    }
-    template <class R> __device__ R rel(int a, double c) const {
-        const double an = (a == 0) ? ax : (a == 1) ? ay : az;
-        const float d = (a == 0) ? dx : (a == 1) ? dy : dz;
-        return static_cast<R>(static_cast<float>(an - c) + d);
     }
     __device__ void drift(float vx, float vy, float vz, double, float d) {
         dx = fmaf(vx, d, dx); dy = fmaf(vy, d, dy); dz = fmaf(vz, d, dz);
@@ -212,7 +249,8 @@ struct PosHL {
     __device__ Snap snap_z() const { return Snap{zh, zl}; }
     __device__ double z_of(Snap s) const { return static_cast<double>(s.h) + static_cast<double>(s.l); }
     __device__ void fold() {}
-    template <class R> __device__ R rel(int a, double c) const {
+    __device__ void refer(const double[3]) {}
+    template <class R> __device__ R at(int a, double c) const {
         const float h = (a == 0) ? xh : (a == 1) ? yh : zh;
         const float l = (a == 0) ? xl : (a == 1) ? yl : zl;
         const float ch = static_cast<float>(c);
@@ -245,6 +283,7 @@ struct Consts {
     R E0[3], G[3];
     double c[3];
     R rfU0, rfV, r0sq;
+    R ir0sq, idm;            // reciprocals for div_by: of r0sq, of the mass (FP64)
     double rfw;
     double acA[2], acw[2], acp[2];   // AC drives (time-dependent field only)
     bool ac;
@@ -284,6 +323,8 @@ __device__ void load_consts(Consts<R>& k, const EnsConst& C, double q, double m)
     k.rfU0 = static_cast<R>(C.rf_U0);
     k.rfV = static_cast<R>(C.rf_V);
     k.r0sq = static_cast<R>(C.r0sq);
+    if constexpr (FIELD == kFieldLinearRF) k.ir0sq = div_reciprocal(k.r0sq);
+    if constexpr (FIELD != kFieldUniform && sizeof(R) == 8) k.idm = div_reciprocal(m);
     k.rfw = C.rf_omega;
     k.ac = C.ac != 0;
 #pragma unroll
@@ -570,11 +611,11 @@ __device__ __forceinline__ void tf_apply(const Consts<R>& k, const TimeField& F,
         float ex = 0.0f, ey = 0.0f, ez = 0.0f;
         const bool local = k.tfc_inst >= 3;   // LQIT, TIMS: x, y from the cylinder axis
         if (f1.y != 0.0f) {          // RF term
-            ex = x.template rel<float>(0, local ? F.ox : 0.0) * f0.x;
-            ey = x.template rel<float>(1, local ? F.oy : 0.0) * f0.y;
+            ex = x.template at<float>(0, local ? F.ox : 0.0) * f0.x;
+            ey = x.template at<float>(1, local ? F.oy : 0.0) * f0.y;
         }
         if (k.tfc_inst == 4) {
-            const float zl = x.template rel<float>(2, F.oz);
+            const float zl = x.template at<float>(2, F.oz);
             tims_segment_sample<R>(k, zl);
             float ei, ef;
             if (k.ts_mode == 2) {
@@ -592,7 +633,7 @@ __device__ __forceinline__ void tf_apply(const Consts<R>& k, const TimeField& F,
         } else if (k.tfc_inst == 3) {
             ex += f0.w;
             ey += f1.x;
-            if (f1.z != 0.0f) ez = (-2.0f * f0.z) * x.template rel<float>(2, F.oz + 0.5 * F.L);
+            if (f1.z != 0.0f) ez = (-2.0f * f0.z) * x.template at<float>(2, F.oz + 0.5 * F.L);
         } else if (f1.z != 0.0f) {
             ez = f0.z;
         }
@@ -603,11 +644,12 @@ __device__ __forceinline__ void tf_apply(const Consts<R>& k, const TimeField& F,
     const bool local = F.inst >= 3;  // LQIT, TIMS: x, y from the cylinder axis
     if (s[1] != 0.0) {
         const double u = s[0];
-        ex = -2.0 * x.template rel<double>(0, local ? F.ox : 0.0) * u / F.r0sq;
-        ey = 2.0 * x.template rel<double>(1, local ? F.oy : 0.0) * u / F.r0sq;
+        const double r0sq = static_cast<double>(k.r0sq), ir0sq = static_cast<double>(k.ir0sq);
+        ex = div_by(-2.0 * x.template at<double>(0, local ? F.ox : 0.0) * u, r0sq, ir0sq);
+        ey = div_by(2.0 * x.template at<double>(1, local ? F.oy : 0.0) * u, r0sq, ir0sq);
     }
     if (F.inst == 4) {
-        const double zl = x.template rel<double>(2, F.oz);
+        const double zl = x.template at<double>(2, F.oz);
         const double f = s[2];
         const double ei = tims_sample(F.tims_z, F.tims_pi, F.tims_nodes, zl, F.tims_ei);
         const double ef = tims_sample(F.tims_z, F.tims_pf, F.tims_final_profile ? F.tims_nodes : 0, zl, F.tims_ef);
@@ -615,7 +657,7 @@ __device__ __forceinline__ void tf_apply(const Consts<R>& k, const TimeField& F,
     } else if (F.inst == 3) {
         ex += s[4];
         ey += s[5];
-        if (s[3] != 0.0) ez = -2.0 * s[2] * (x.template rel<double>(2, F.oz) - 0.5 * F.L);
+        if (s[3] != 0.0) ez = -2.0 * s[2] * (x.template at<double>(2, F.oz) - 0.5 * F.L);
     } else if (s[3] != 0.0) {
         ez = s[2];
     }
@@ -623,28 +665,66 @@ __device__ __forceinline__ void tf_apply(const Consts<R>& k, const TimeField& F,
 }
 
 #ifdef ICB_TF_TABLE_UNIT
-// Per-step scalars of the launch for the ensembles with a time-dependent
-// field (built in the FP64 unit only, without FMA contraction, for every
-// precision): block e fills rows k = 0..K of the table of chunk ensemble e
-// (global index ens_base + e; stage 0 at t_k, stage 1 at t_k + dt/2 for
-// RK4), t_k accumulated as the step kernel does (t_{k+1} = t_k + dt) into
-// tseq first, so each lane reads the values it would compute.
+// t_{k+1} = t_k + dt, k < n, accumulated in floating point, by one block.
+// While t stays in one binade the rounded increment is the same every step,
+// so t_k + j d with d = (t_k + dt) - t_k is the sequence: thread j proposes
+// that value and checks the recurrence against its predecessor's, the steps
+// before the first that fails are accepted, and the next round starts there
+// (its first step is the plain sum, so every round advances; a round ends at
+// a binade's end or a tie).  put(k, t_k) receives every value, k = 0..n, and
+// the last is returned to every thread.  A serial loop of 1,000 sums took
+// 7 us, 16 us with its stores.
+template <class Put>
+__device__ double clock_sequence(double t0, double dt, uint32_t n, Put put) {
+    const uint32_t j = threadIdx.x;
+    if (j == 0) put(0u, t0);
+    double base = t0;
+    uint32_t k = 0;
+    __shared__ uint32_t first_bad;
+    __shared__ double next_base;
+    while (k < n) {
+        const uint32_t m = min(n - k, static_cast<uint32_t>(blockDim.x));
+        const double d = (base + dt) - base;
+        auto cand = [&](uint32_t i) { return i == 0u ? base + dt : fma(static_cast<double>(i + 1u), d, base); };
+        const double c = cand(j);
+        const bool ok = j == 0u || (j < m && cand(j - 1u) + dt == c);
+        if (j == 0) first_bad = m;
+        __syncthreads();
+        const unsigned bad = __ballot_sync(0xffffffffu, !ok);
+        if ((j & 31u) == 0u && bad) atomicMin(&first_bad, j + static_cast<uint32_t>(__ffs(static_cast<int>(bad))) - 1u);
+        __syncthreads();
+        const uint32_t acc = min(first_bad, m);          // accepted: j < acc
+        if (j < acc) put(k + j + 1u, c);
+        if (j == acc - 1u) next_base = c;
+        __syncthreads();
+        base = next_base;
+        k += acc;
+        __syncthreads();
+    }
+    return base;
+}
+
+// Per-step scalars of the launch for the ensembles whose field depends on
+// time only through them (built in the FP64 unit only, without FMA
+// contraction, for every precision; the trap with RF and two AC drives spent
+// half its step on the three double cosines of every lane: 100,001 ions, 500
+// steps, 1910 -> 1234 us).  Block e fills rows k = 0..K of the
+// table of chunk ensemble e (global index ens_base + e; stage 0 at t_k,
+// stage 1 at t_k + dt/2 for RK4), t_k accumulated as the step kernel does,
+// so each lane reads the values it would compute.  Waveform and TIMS
+// ensembles: tf_scalars.  Constant-voltage RF and AC drives: cos(w t) of the
+// RF and the two drives' a cos(w t + phase) (their phase sum contracted as
+// the float units contract it).
 __global__ void k_tf_table(const StepParams p, double* tab, double* tseq, uint32_t stride) {
     const uint32_t e = blockIdx.x;
     const EnsConst& C = p.ens[e];
-    if (!C.tf) return;
+    if (!C.tf && !C.rf && !C.ac) return;
     const uint32_t g = p.ens_base + e;
-    const TimeField& F = p.tfield[g];
+    const TimeField* F = C.tf ? p.tfield + g : nullptr;
     const uint32_t rows = p.n_steps + 1u;
     double* T = tab + static_cast<size_t>(g) * rows * stride;
     double* ts = tseq + static_cast<size_t>(g) * rows;
-    if (threadIdx.x == 0) {
-        double t = p.t_dev[g];
-        for (uint32_t k = 0; k < rows; ++k) {
-            ts[k] = t;
-            t = t + C.dt;
-        }
-    }
+    clock_sequence(p.t_dev[g], C.dt, p.n_steps, [&](uint32_t k, double t) { ts[k] = t; });
     __syncthreads();
     const double hd = C.dt * 0.5;
     for (uint32_t k = threadIdx.x; k < rows; k += blockDim.x) {
@@ -663,17 +743,64 @@ __global__ void k_tf_table(const StepParams p, double* tab, double* tseq, uint32
             f[6] = sc[3] != 0.0 ? 1.0f : 0.0f;
             f[7] = 0.0f;
         };
-        tf_scalars(F, t, sc);
-        put(row);
+        auto drives = [&](double* r, double tt) {
+            r[0] = C.rf ? cos(C.rf_omega * tt) : 0.0;
+            r[1] = r[2] = 0.0;
+            if (C.ac) {
+                for (int a = 0; a < 2; ++a) {
+                    const double ph = p.tab_fused ? fma(C.ac_omega[a], tt, C.ac_phase[a])
+                                                  : C.ac_omega[a] * tt + C.ac_phase[a];
+                    r[1 + a] = C.ac_amp[a] * cos(ph);
+                }
+            }
+            float* f = reinterpret_cast<float*>(r + kTfScalars);
+            for (int j = 0; j < 3; ++j) f[j] = static_cast<float>(r[j]);
+        };
+        if (F) {
+            tf_scalars(*F, t, sc);
+            put(row);
+        } else {
+            drives(row, t);
+        }
         if (stride > static_cast<uint32_t>(kTfRowScalars)) {
-            tf_scalars(F, t + hd, sc);
-            put(row + kTfRowScalars);
+            if (F) {
+                tf_scalars(*F, t + hd, sc);
+                put(row + kTfRowScalars);
+            } else {
+                drives(row + kTfRowScalars, t + hd);
+            }
         }
     }
+}
+
+// Device engine clock: step += K and t_e += dt_e, K times (accumulated like
+// the engine's per-step t += dt, SimulationEngineLifecycle.cpp:162).  One
+// block per ensemble.
+__global__ void __launch_bounds__(256) k_clock_advance(unsigned long long* step, double* t, const double* dt,
+                                                       uint32_t K) {
+    const uint32_t e = blockIdx.x;
+    if (e == 0 && threadIdx.x == 0) *step += K;
+    const double end = clock_sequence(t[e], dt[e], K, [](uint32_t, double) {});
+    if (threadIdx.x == 0) t[e] = end;
 }
 #endif
 
 // ---- fields -----------------------------------------------------------------
+// The drives' cosines of a launch too short for a table (out of line: the
+// table's readers keep their registers).
+static __device__ __noinline__ double rf_cos(double w, double t) { return cos(w * t); }
+static __device__ __noinline__ double ac_drive(double a, double w, double t, double phase) {
+    return a * cos(w * t + phase);
+}
+
+// Scalar j of a table row in the working precision (the float block holds
+// the doubles rounded once).
+template <class R>
+__device__ __forceinline__ R row_value(const double* row, int j) {
+    if constexpr (sizeof(R) == 4) return reinterpret_cast<const float*>(row + kTfScalars)[j];
+    else return row[j];
+}
+
 template <class R, int FIELD, class Pos>
 __device__ __forceinline__ void efield(const Consts<R>& k, const Pos& x, double t, R E[3], int stage = 0) {
     if constexpr (FIELD == kFieldUniform) {
@@ -681,7 +808,7 @@ __device__ __forceinline__ void efield(const Consts<R>& k, const Pos& x, double 
         return;
     } else if constexpr (FIELD == kFieldLinear) {
 #pragma unroll
-        for (int a = 0; a < 3; ++a) E[a] = k.E0[a] + k.G[a] * x.template rel<R>(a, k.c[a]);
+        for (int a = 0; a < 3; ++a) E[a] = k.E0[a] + k.G[a] * x.template at<R>(a, k.c[a]);
         return;
     } else {
         if (k.tf != nullptr) {
@@ -691,23 +818,27 @@ __device__ __forceinline__ void efield(const Consts<R>& k, const Pos& x, double 
             return;
         } else {
 #pragma unroll
-            for (int a = 0; a < 3; ++a) E[a] = k.E0[a] + k.G[a] * x.template rel<R>(a, k.c[a]);
+            for (int a = 0; a < 3; ++a) E[a] = k.E0[a] + k.G[a] * x.template at<R>(a, k.c[a]);
             // AnalyticalFieldModel.cpp:152-158: U = dc_quad + V cos(w t);
             // E_x = -2 x U / r0^2, E_y = 2 y U / r0^2, x and y from the
             // quadrupole axis (c[0], c[1]: 0 for IMS / QuadrupoleRF, the
             // cylinder axis for the LQIT, AnalyticalFieldModel.cpp:90-103).
             // Without an RF voltage the LQIT's x, y come from G = 0.
+            // The time-only cosines come from the launch's table (k_tf_table)
+            // when it has one; a launch of a few steps evaluates them here.
+            const double* row = k.tftab == nullptr ? nullptr : k.tfrow +
+                (stage == 0 ? 0 : stage == 1 ? kTfRowScalars : static_cast<int>(k.tfstride));
             if (k.rfV != R(0)) {
-                const R U = k.rfU0 + k.rfV * static_cast<R>(cos(k.rfw * t));
-                const R px = x.template rel<R>(0, k.c[0]), py = x.template rel<R>(1, k.c[1]);
-                E[0] = R(-2.0) * px * U / k.r0sq;
-                E[1] = R(2.0) * py * U / k.r0sq;
+                const R U = k.rfU0 + k.rfV * (row ? row_value<R>(row, 0) : static_cast<R>(rf_cos(k.rfw, t)));
+                const R px = x.template at<R>(0, k.c[0]), py = x.template at<R>(1, k.c[1]);
+                E[0] = div_by(R(-2.0) * px * U, k.r0sq, k.ir0sq);
+                E[1] = div_by(R(2.0) * py * U, k.r0sq, k.ir0sq);
             }
-        }
-        // LQIT AC drives (AnalyticalFieldModel.cpp:104-121)
-        if (k.ac) {
-            E[0] += static_cast<R>(k.acA[0] * cos(k.acw[0] * t + k.acp[0]));
-            E[1] += static_cast<R>(k.acA[1] * cos(k.acw[1] * t + k.acp[1]));
+            // LQIT AC drives (AnalyticalFieldModel.cpp:104-121)
+            if (k.ac) {
+                E[0] += row ? row_value<R>(row, 1) : static_cast<R>(ac_drive(k.acA[0], k.acw[0], t, k.acp[0]));
+                E[1] += row ? row_value<R>(row, 2) : static_cast<R>(ac_drive(k.acA[1], k.acw[1], t, k.acp[1]));
+            }
         }
     }
 }
@@ -727,10 +858,10 @@ __device__ __forceinline__ R boris(const Consts<R>& k, Pos& x, R v[3], double t)
         if constexpr (sizeof(R) == 8) {
             if (k.sc) {
 #pragma unroll
-                for (int c = 0; c < 3; ++c) a[c] = (E[c] * k.q + k.escq[c]) / static_cast<R>(k.m);
+                for (int c = 0; c < 3; ++c) a[c] = div_by(E[c] * k.q + k.escq[c], k.m, k.idm);
             } else {
 #pragma unroll
-                for (int c = 0; c < 3; ++c) a[c] = (E[c] * k.q) / static_cast<R>(k.m);
+                for (int c = 0; c < 3; ++c) a[c] = div_by(E[c] * k.q, k.m, k.idm);
             }
         } else {
             if (k.sc) {
@@ -1392,11 +1523,15 @@ __global__ void __launch_bounds__(128, KernelShape<PREC, COLL, FIELD>::kMinBlock
     k.tfrow = nullptr;
     k.tfstride = p.tf_stride;
     if constexpr (FIELD == kFieldLinearRF) {
-        if (C.tf && p.tfield != nullptr && p.tf_tab != nullptr) {
-            k.tf = p.tfield + (p.ens_base + static_cast<uint32_t>(e));
+        if (C.tf && p.tfield != nullptr && p.tf_tab != nullptr) k.tf = p.tfield + (p.ens_base + static_cast<uint32_t>(e));
+        if (p.tf_tab != nullptr && (C.tf || ((C.rf || C.ac) && p.rf_tab))) {
             k.tftab = p.tf_tab + static_cast<size_t>(p.ens_base + static_cast<uint32_t>(e)) * (p.n_steps + 1u) *
                                      p.tf_stride;
             k.tfrow = k.tftab;
+        }
+        if (k.tf != nullptr) {
+            k.r0sq = static_cast<R>(k.tf->r0sq);
+            k.ir0sq = div_reciprocal(k.r0sq);
             if constexpr (sizeof(R) == 4) {
                 const TimeField& F = *k.tf;
                 k.tfc_inst = F.inst;
@@ -1505,6 +1640,26 @@ __global__ void __launch_bounds__(128, KernelShape<PREC, COLL, FIELD>::kMinBlock
     Snap zold{};
     R acc = R(0), lim = R(0);
 
+    // Reference point of the field's position terms (PosA::at): the field's
+    // centre, or for the time-dependent field the point tf_apply names.
+    auto refer = [&]() {
+        if constexpr (FIELD != kFieldUniform && PREC == kPrecMixed) {
+            double c[3] = {C.c[0], C.c[1], C.c[2]};
+            if (FIELD == kFieldLinearRF && k.tf != nullptr) {
+                const bool local = k.tfc_inst >= 3;
+                c[0] = local ? C.ox : 0.0;
+                c[1] = local ? C.oy : 0.0;
+                c[2] = k.tfc_inst == 3 ? C.oz + 0.5 * k.tf->L : C.oz;
+            }
+            x.refer(c);
+        }
+    };
+    refer();
+    auto fold = [&]() {
+        x.fold();
+        refer();
+    };
+
     auto t_step = [&]() -> double { return kAccumT ? t : fma(static_cast<double>(kk), dt, t0); };
     // z component of the parabolic gas flow at the ion
     // (EnvironmentConfig::gas_velocity_at, EnvironmentConfig.h:115-125)
@@ -1577,7 +1732,7 @@ __global__ void __launch_bounds__(128, KernelShape<PREC, COLL, FIELD>::kMinBlock
         if (do_fin && (!FUSED || !(acc <= lim))) {
             double zo = x.z_of(zold);
             if (!FUSED && !do_push) zo = p.zprev[i];
-            x.fold();
+            fold();
             check_exact(zo, t_step());
         }
         ++kk;
@@ -1666,7 +1821,7 @@ __global__ void __launch_bounds__(128, KernelShape<PREC, COLL, FIELD>::kMinBlock
             double tn = 0.0;   // only a time-dependent field reads the clock
             if constexpr (FIELD == kFieldLinearRF) {
                 tn = t_step();
-                if (k.tf != nullptr) k.tfrow = k.tftab + static_cast<size_t>(kk) * k.tfstride;
+                if (k.tftab != nullptr) k.tfrow = k.tftab + static_cast<size_t>(kk) * k.tfstride;
             }
             if (INTEG == kBoris) l1 = boris<R, FIELD, MAG>(k, x, v, tn);
             else l1 = rk4<R, FIELD, MAG>(k, x, v, tn);
@@ -1737,7 +1892,7 @@ __global__ void __launch_bounds__(128, KernelShape<PREC, COLL, FIELD>::kMinBlock
             }
             // warp-uniform fold of the float position offsets (anchor mode);
             // pending lanes keep theirs until their step is finalized
-            if (!pending) x.fold();
+            if (!pending) fold();
             const bool can_step = (kBirths ? (live || waiting) : live) && !pending && kk < K;
             const unsigned pend_mask = __ballot_sync(0xffffffffu, pending);
             const unsigned run_mask = __ballot_sync(0xffffffffu, can_step);
