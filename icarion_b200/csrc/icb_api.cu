@@ -339,6 +339,7 @@ struct icb_handle {
     std::vector<icb_tims_field> tims;
     std::vector<uint8_t> tims_set;
     DevBuf<TimeField> tfield;
+    const double2* cs_tab = nullptr;   // FP64 collisions: functions of the 16-bit draws
     DevBuf<double> tf_tab;             // per-step field scalars, one launch chunk at a time
     bool any_tf = false;
     int base_field_kind = kFieldUniform;
@@ -905,6 +906,7 @@ int launch_step(icb_handle* h, uint32_t K, int do_push, int do_collide, int do_f
         p.ehss_atoms = h->ehss_atoms.p;
         p.ehss_off = h->ehss_off.p;
         p.ehss_rgas = h->ehss_rgas.p;
+        p.cs_tab = h->cs_tab;
         p.counters = h->counters.p;
         p.step_dev = h->step_dev.p;
         p.t_dev = h->t_dev.p;
@@ -1190,6 +1192,18 @@ int icb_create(const icb_config* cfg, icb_handle** out) {
     // Deferred-collision batch per warp (lanes of 32): measured optimum with
     // 8 steps per vote.
     h->pend = 10u;
+    // The planned FP64 loop (uniform field, no B): its steps are cheap next to
+    // its events, so the warp votes every 16 steps, and waits for 16 pending
+    // lanes where events are frequent (A <|th|> per step).  262,144 ions x
+    // 1,000 steps, pending / vote: at 1000 Pa (0.085) 10/8 3050 us, 16/16
+    // 2677, 24/16 2678; at 100 Pa (0.0085) 1007, 881 (10/16 879); at 30 Pa
+    // 689, 717, 947 (10/16 619).
+    if (h->fp64() && cfg->integrator == ICB_INTEGRATOR_BORIS && h->field_kind == kFieldUniform && !h->magnetic) {
+        double rate = 0.0;
+        for (const EnsConst& c : h->ens_const) rate = std::max(rate, c.A * c.mean_th);
+        h->spv = 16u;
+        if (rate >= 0.01) h->pend = 16u;
+    }
     if (cfg->pending_threshold > 0) h->pend = static_cast<uint32_t>(std::min(cfg->pending_threshold, 32));
     if (cfg->steps_per_vote > 0) h->spv = static_cast<uint32_t>(std::min(cfg->steps_per_vote, 64));
     if (cfg->stepping != ICB_STEPPING_EVENTS && cfg->stepping != ICB_STEPPING_PER_STEP &&
@@ -1362,6 +1376,8 @@ int icb_upload_ions(icb_handle* h, uint64_t n,
     if (birth_time_s) ICB_CUDA(cudaMemcpyAsync(h->birth.p, birth_time_s, bytes, cudaMemcpyHostToDevice, s));
     k_flags_in<<<g, 256, 0, s>>>(h->active_stage.p, h->has_birth ? h->birth.p : nullptr, h->flags.p, h->t_death.p, h->t_arr.p, n);
     ICB_CUDA(cudaGetLastError());
+    if (h->fp64() && h->coll != kCollNone && h->coll != kCollHSSPlain)
+        ICB_CUDA(launch_angle_table(&h->cs_tab, s));
     if (h->coll != kCollNone) {
         const int skip = h->skip_clock() ? 1 : 0;
         if (h->fp64())

@@ -14,6 +14,9 @@ namespace icb {
 // launch's cudaError_t (cudaErrorNotSupported for an absent combination).
 // Per-step time-only field scalars of one launch (tf_tab of StepParams).
 cudaError_t launch_tf_table(const StepParams& p, double* tab, double* tseq, uint32_t stride, cudaStream_t s);
+// The FP64 forms' table of functions of a 16-bit draw on the current device
+// (1.5 MB of module memory), filled on `s` where it is not yet.
+cudaError_t launch_angle_table(const double2** tab, cudaStream_t s);
 // The device engine clock K steps on (step_dev, t_dev).
 cudaError_t launch_clock_advance(unsigned long long* step, double* t, const double* dt, int n_ens, uint32_t K,
                                  cudaStream_t s);

@@ -193,6 +193,7 @@ struct StepParams {
     const double4* ehss_atoms;
     const int32_t* ehss_off;
     const double* ehss_rgas;
+    const double2* cs_tab;             // FP64: functions of the 65,536 16-bit draws
     unsigned long long* counters;      // kNumCounters
     const unsigned long long* step_dev;// engine step index at launch start
     const double* t_dev;               // engine time per ensemble at launch start

@@ -17,6 +17,15 @@ cudaError_t launch_tf_table(const StepParams& p, double* tab, double* tseq, uint
     return cudaGetLastError();
 }
 
+cudaError_t launch_angle_table(const double2** tab, cudaStream_t s) {
+    void* p = nullptr;
+    const cudaError_t e = cudaGetSymbolAddress(&p, g_angle_tab);
+    if (e != cudaSuccess) return e;
+    *tab = static_cast<const double2*>(p);
+    k_angle_table<<<kAngles / 256, 256, 0, s>>>();
+    return cudaGetLastError();
+}
+
 cudaError_t launch_clock_advance(unsigned long long* step, double* t, const double* dt, int n_ens, uint32_t K,
                                  cudaStream_t s) {
     // a launch of few steps needs no more than a warp

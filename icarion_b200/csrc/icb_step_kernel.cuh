@@ -148,6 +148,47 @@ __device__ __forceinline__ void angle_cs(float u, float& c, float& s) {
     __sincosf(6.28318530717958648f * (u - 0.5f), &s, &c);
 }
 
+// Functions of a 16-bit draw k: (cos, sin) of (k + 1/2) 2^-16 of a turn, and
+// sqrt(1 - c^2) of the polar cosine c = 2 (k + 1/2) 2^-16 - 1.  FP64 reads
+// both from a table of all 65,536 draws filled by the expressions below, so
+// the same values; three pairs and two roots a candidate were over half its
+// double operations.
+constexpr uint32_t kAngles = 65536u;
+constexpr uint32_t kAngleTab = kAngles + kAngles / 2u;     // double2: the pairs, then the roots two by two
+__device__ __forceinline__ void angle16(uint32_t k, const double2* tab, double& c, double& s) {
+    const double2 v = __ldg(tab + k);
+    c = v.x;
+    s = v.y;
+}
+__device__ __forceinline__ void angle16(uint32_t k, const double2*, float& c, float& s) {
+    angle_cs(u16(k, 0.0f), c, s);
+}
+__device__ __forceinline__ double polar_sin(double ct) { return m_sqrt(m_fmax(0.0, 1.0 - ct * ct)); }
+__device__ __forceinline__ double polar16(uint32_t k, double, const double2* tab) {
+    return __ldg(reinterpret_cast<const double*>(tab + kAngles) + k);
+}
+__device__ __forceinline__ float polar16(uint32_t, float ct, const double2*) {
+    return m_sqrt(m_fmax(0.0f, 1.0f - ct * ct));
+}
+#ifdef ICB_TF_TABLE_UNIT
+__device__ double2 g_angle_tab[kAngleTab];
+// Fills the entries that are still zero (no filled pair is): every upload of
+// an FP64 handle runs it on its own stream, so the table is there whatever
+// other handles or device resets did, and is never rewritten under a reader.
+__global__ void k_angle_table() {
+    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= kAngles) return;
+    const double2 old = g_angle_tab[k];
+    if (old.x != 0.0 || old.y != 0.0) return;
+    const double ct = 2.0 * u16(k, 0.0) - 1.0;
+    reinterpret_cast<double*>(g_angle_tab + kAngles)[k] = polar_sin(ct);
+    __threadfence();
+    double c, s;
+    angle_cs(u16(k, 0.0), c, s);
+    g_angle_tab[k] = make_double2(c, s);
+}
+#endif
+
 // ---- positions --------------------------------------------------------------
 // Double position (FP64).
 struct PosD {
@@ -1216,14 +1257,14 @@ __device__ __forceinline__ int candidate(const EnsConst& C, R v[3], R& clk, R qs
     // Langevin capture: Maxwellian neutral (the thermal branch), every event collides
     const bool thermal = LANG || (uc * (b + mean_th) < b);
     R c3, s3;
-    angle_cs(u16(r1.y >> 16, R(0)), c3, s3);
+    angle16(r1.y >> 16, p.cs_tab, c3, s3);
     const R sfac = thermal ? c3 * c3 : R(1);
     const R r2 = R(-2.0) * (m_log(u32(r0.w, R(0))) + m_log(u32(r1.x, R(0))) * sfac);
     const R rad = sig_n * m_sqrt(r2);
     const R ct = R(2.0) * u16(r1.y & 0xffffu, R(0)) - R(1.0);
-    const R st = m_sqrt(m_fmax(R(0), R(1.0) - ct * ct));
+    const R st = polar16(r1.y & 0xffffu, ct, p.cs_tab);
     R cp, sp;
-    angle_cs(u16(r1.z >> 16, R(0)), cp, sp);
+    angle16(r1.z >> 16, p.cs_tab, cp, sp);
     const R vn[3] = {ug[0] + rad * (st * cp), ug[1] + rad * (st * sp), ug[2] + rad * ct};
     const R gx = v[0] - vn[0], gy = v[1] - vn[1], gz = v[2] - vn[2];
     const R g = m_sqrt(gx * gx + gy * gy + gz * gz);
@@ -1243,7 +1284,7 @@ __device__ __forceinline__ int candidate(const EnsConst& C, R v[3], R& clk, R qs
         const R mu = mi * fac;   // m_i m_n / (m_i + m_n); the product m_i m_n underflows in float
         ip->E = R(0.5) * mu * (g * g);
         ip->bn = m_sqrt(u16(r1.z & 0xffffu, R(0)));
-        angle_cs(u16(r1.w >> 16, R(0)), ip->cp, ip->sp);
+        angle16(r1.w >> 16, p.cs_tab, ip->cp, ip->sp);
         ip->g3[0] = gx; ip->g3[1] = gy; ip->g3[2] = gz;
         ip->g = g;
         ip->vn[0] = vn[0]; ip->vn[1] = vn[1]; ip->vn[2] = vn[2];
@@ -1264,7 +1305,7 @@ __device__ __forceinline__ int candidate(const EnsConst& C, R v[3], R& clk, R qs
             cx = ipm_table_cos<R>(p, E, bn);
         const R sx = m_sqrt(m_fmax(R(0), R(1) - cx * cx));
         R cp2, sp2;
-        angle_cs(u16(r1.w >> 16, R(0)), cp2, sp2);
+        angle16(r1.w >> 16, p.cs_tab, cp2, sp2);
         const R g3[3] = {gx, gy, gz};
         R gp[3];
         deflect<R>(g3, g, cx, sx, cp2, sp2, gp);
@@ -1276,9 +1317,9 @@ __device__ __forceinline__ int candidate(const EnsConst& C, R v[3], R& clk, R qs
         return 2;
     }
     const R ct2 = R(2.0) * u16(r1.z & 0xffffu, R(0)) - R(1.0);
-    const R st2 = m_sqrt(m_fmax(R(0), R(1.0) - ct2 * ct2));
+    const R st2 = polar16(r1.z & 0xffffu, ct2, p.cs_tab);
     R cp2, sp2;
-    angle_cs(u16(r1.w >> 16, R(0)), cp2, sp2);
+    angle16(r1.w >> 16, p.cs_tab, cp2, sp2);
     const R dir[3] = {st2 * cp2, st2 * sp2, ct2};
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -1301,7 +1342,7 @@ __device__ __forceinline__ int candidate(const EnsConst& C, R v[3], R& clk, R qs
 template <class R, bool SKIP>
 __device__ __forceinline__ int candidate_mix(const EnsConst& C, const MixConst& M, R v[3], R& clk, R qstar,
                                              R Amean, R b, double mi_d, const uint32_t* rk, uint32_t id,
-                                             uint32_t step, const PhiloxIon& pq) {
+                                             uint32_t step, const PhiloxIon& pq, const StepParams& p) {
     constexpr bool D = sizeof(R) == 8;
     R ug[3], mi;
     if constexpr (D) {
@@ -1345,14 +1386,14 @@ __device__ __forceinline__ int candidate_mix(const EnsConst& C, const MixConst& 
     const U4 r1 = philox_ion(pq, step, 1u, rk);
     const bool thermal = uci * (b + Mi(ci)) < b;
     R c3, s3;
-    angle_cs(u16(r1.y >> 16, R(0)), c3, s3);
+    angle16(r1.y >> 16, p.cs_tab, c3, s3);
     const R sfac = thermal ? c3 * c3 : R(1);
     const R r2 = R(-2.0) * (m_log(u32(r0.w, R(0))) + m_log(u32(r1.x, R(0))) * sfac);
     const R rad = Si(ci) * m_sqrt(r2);
     const R ct = R(2.0) * u16(r1.y & 0xffffu, R(0)) - R(1.0);
-    const R st = m_sqrt(m_fmax(R(0), R(1.0) - ct * ct));
+    const R st = polar16(r1.y & 0xffffu, ct, p.cs_tab);
     R cp, sp;
-    angle_cs(u16(r1.z >> 16, R(0)), cp, sp);
+    angle16(r1.z >> 16, p.cs_tab, cp, sp);
     const R vn[3] = {ug[0] + rad * (st * cp), ug[1] + rad * (st * sp), ug[2] + rad * ct};
     const R gx = v[0] - vn[0], gy = v[1] - vn[1], gz = v[2] - vn[2];
     const R g = m_sqrt(gx * gx + gy * gy + gz * gz);
@@ -1363,8 +1404,8 @@ __device__ __forceinline__ int candidate_mix(const EnsConst& C, const MixConst& 
         const R ra = m_sqrt(R(-2.0) * m_log(u32(rj.x, R(0))));
         const R rb = m_sqrt(R(-2.0) * m_log(u32(rj.y, R(0))));
         R ca, sa, cb2, sb2;
-        angle_cs(u16(rj.z >> 16, R(0)), ca, sa);
-        angle_cs(u16(rj.z & 0xffffu, R(0)), cb2, sb2);
+        angle16(rj.z >> 16, p.cs_tab, ca, sa);
+        angle16(rj.z & 0xffffu, p.cs_tab, cb2, sb2);
         const R s = Si(j);
         const R hx = v[0] - (ug[0] + s * ra * ca);
         const R hy = v[1] - (ug[1] + s * ra * sa);
@@ -1379,9 +1420,9 @@ __device__ __forceinline__ int candidate_mix(const EnsConst& C, const MixConst& 
     else inv_mt = __frcp_rn(mi + mn);
     const R fac = mn * inv_mt;
     const R ct2 = R(2.0) * u16(r1.z & 0xffffu, R(0)) - R(1.0);
-    const R st2 = m_sqrt(m_fmax(R(0), R(1.0) - ct2 * ct2));
+    const R st2 = polar16(r1.z & 0xffffu, ct2, p.cs_tab);
     R cp2, sp2;
-    angle_cs(u16(r1.w >> 16, R(0)), cp2, sp2);
+    angle16(r1.w >> 16, p.cs_tab, cp2, sp2);
     const R dir[3] = {st2 * cp2, st2 * sp2, ct2};
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -1758,7 +1799,7 @@ __global__ void __launch_bounds__(128, KernelShape<PREC, COLL, FIELD>::kMinBlock
                     if (p.flows && C.flow) { v[2] = v[2] - flow_z(); shifted = true; }
                     int st;
                     if constexpr (COLL == kCollHSSMix)
-                        st = candidate_mix<R, true>(C, p.mix[p.ens_base + e], v, S, U, k.Amean, b, m, p.rk, id, gs, pq);
+                        st = candidate_mix<R, true>(C, p.mix[p.ens_base + e], v, S, U, k.Amean, b, m, p.rk, id, gs, pq, p);
                     else
                         st = candidate<R, true, COLL>(C, v, S, U, k.Amean, b, m, p.rk, id, gs, p, &ip, p.ens_base + e, pq);
                     if (st >= 1) ++n_cand;
@@ -1770,7 +1811,7 @@ __global__ void __launch_bounds__(128, KernelShape<PREC, COLL, FIELD>::kMinBlock
                 ++n_cand;
                 int st;
                 if constexpr (COLL == kCollHSSMix)
-                    st = candidate_mix<R, false>(C, p.mix[p.ens_base + e], v, U, R(0), k.Amean, b, m, p.rk, id, gs, pq);
+                    st = candidate_mix<R, false>(C, p.mix[p.ens_base + e], v, U, R(0), k.Amean, b, m, p.rk, id, gs, pq, p);
                 else
                     st = candidate<R, false, COLL>(C, v, U, R(0), k.Amean, b, m, p.rk, id, gs, p, &ip, p.ens_base + e, pq);
                 if (st >= 2) ++n_coll;
@@ -1896,8 +1937,10 @@ __global__ void __launch_bounds__(128, KernelShape<PREC, COLL, FIELD>::kMinBlock
             const bool can_step = (kBirths ? (live || waiting) : live) && !pending && kk < K;
             const unsigned pend_mask = __ballot_sync(0xffffffffu, pending);
             const unsigned run_mask = __ballot_sync(0xffffffffu, can_step);
-            if (pend_mask != 0u &&
-                (run_mask == 0u || static_cast<uint32_t>(__popc(pend_mask)) >= p.pend_threshold)) {
+            // without collisions a stopped lane has only its exact check to make:
+            // FP64 (whose results do not depend on when) makes it at once
+            const uint32_t thr = (PREC == kPrecFP64 && COLL == kCollNone) ? 1u : p.pend_threshold;
+            if (pend_mask != 0u && (run_mask == 0u || static_cast<uint32_t>(__popc(pend_mask)) >= thr)) {
                 collide_at(pending && cand, step0 + kk);
                 if (pending) {
                     cand = false;
@@ -1984,10 +2027,98 @@ __global__ void __launch_bounds__(128, KernelShape<PREC, COLL, FIELD>::kMinBlock
             if (exact) check_exact(zo, fma(static_cast<double>(kk - 1u), dt, t0));
         }
     };
+    // FP64 in a uniform field without B, step by step in the reference's
+    // operation order (the loop above with its bookkeeping planned ahead).
+    // The steps up to a lane's next stop are known before they are taken: its
+    // clock event, the launch end, or the step at which the displacement
+    // budget may run out (run_jumps' bound B).  The pushes between are 13
+    // double operations without tests; a stop leaves the lane pending as
+    // above.  One ion's chain of steps bounds a small population and the
+    // double pipe a large one.
+    auto run_tight = [&]() {
+        const R a0 = k.a_uni[0], a1 = k.a_uni[1], a2 = k.a_uni[2];
+        const R ca = (m_fabs(a0) + m_fabs(a1) + m_fabs(a2)) * dt_r * dt_r;
+        const R ah0 = a0 * k.h, ah1 = a1 * k.h, ah2 = a2 * k.h;
+        const uint32_t thr = COLL == kCollNone ? 1u : p.pend_threshold;
+        uint32_t left = 0;            // pushes of the plan not yet taken
+        bool ev = false, stop = false;
+        auto push = [&]() {
+            v[0] = v[0] + ah0; v[1] = v[1] + ah1; v[2] = v[2] + ah2;
+            x.drift(v[0], v[1], v[2], dt, dt_r);
+            v[0] = v[0] + ah0; v[1] = v[1] + ah1; v[2] = v[2] + ah2;
+        };
+        while (true) {
+            if (live && !pending && kk < K) {
+                if (left == 0u) {
+                    uint32_t n = K - kk, ne = 0xFFFFFFFFu;
+                    if constexpr (kSkip) {
+                        ne = nk + 1u - kk;
+                        if (ne < n) n = ne;
+                    }
+                    const R sd = (m_fabs(v[0] + ah0) + m_fabs(v[1] + ah1) + m_fabs(v[2] + ah2)) * dt_r;
+                    auto bound = [&](uint32_t j) {
+                        const R rj = static_cast<R>(j);
+                        return rj * (sd + R(0.5) * ca * (rj - R(1)));
+                    };
+                    const R rem = lim - acc;
+                    if (!(bound(n) <= rem)) {
+                        uint32_t nb = 0;
+                        if (rem >= R(0)) {
+                            const R B = sd - R(0.5) * ca;
+                            const R den = B + m_sqrt(m_fmax(B * B + R(2) * ca * rem, R(0)));
+                            R nbf = R(0);
+                            if (den > R(0)) nbf = (R(2) * rem) / den;
+                            else if (den == R(0)) nbf = static_cast<R>(n);
+                            nb = nbf >= static_cast<R>(n) ? n : static_cast<uint32_t>(nbf);
+                            if (nb > 0u && !(bound(nb) <= rem)) --nb;
+                        }
+                        if (nb + 1u < n) n = nb + 1u;
+                    }
+                    ev = n == ne;
+                    acc += bound(n);
+                    stop = ev || !(acc <= lim);
+                    left = n;
+                }
+                const uint32_t m = left < p.steps_per_vote ? left : p.steps_per_vote;
+                left -= m;
+                const bool last = stop && left == 0u;
+                const uint32_t free_steps = last ? m - 1u : m;
+#pragma unroll 4
+                for (uint32_t j = 0; j < free_steps; ++j) {
+                    push();
+                    t = t + dt;
+                }
+                kk += free_steps;
+                if (last) {
+                    zold = x.snap_z();
+                    push();
+                    pending = true;
+                    cand = ev;
+                }
+            }
+            const bool can_step = live && !pending && kk < K;
+            const unsigned pend_mask = __ballot_sync(0xffffffffu, pending);
+            const unsigned run_mask = __ballot_sync(0xffffffffu, can_step);
+            if (pend_mask != 0u && (run_mask == 0u || static_cast<uint32_t>(__popc(pend_mask)) >= thr)) {
+                collide_at(pending && cand, step0 + kk);
+                if (pending) {
+                    cand = false;
+                    pending = false;
+                    finalize_step();
+                }
+                continue;
+            }
+            if (run_mask == 0u) break;
+        }
+    };
     if (__any_sync(0xffffffffu, waiting)) {
         run(std::true_type{});
     } else {
-        if constexpr (kJump) {
+        if constexpr (kJump && PREC == kPrecFP64) {
+            if (p.jumps) run_jumps();
+            else if (budget) run_tight();
+            else run(std::false_type{});
+        } else if constexpr (kJump) {
             if (p.jumps) run_jumps();
             else run(std::false_type{});
         } else {
