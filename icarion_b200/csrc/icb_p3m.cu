@@ -374,21 +374,30 @@ __global__ void k_sc_cmul_fold(MeshGeom g, const cufftComplex* __restrict__ a, c
 }
 
 // ---------------------------------------------------------------------------
-// Fused x pass of the single-precision mesh for a padded x length of 256 (a
-// 128-node mesh axis).  Per (ky, kz) column of the 2D-transformed mesh
-// planes: the forward 256-point transform along x (inputs x >= 128 are the
-// zero padding), the products with i G_c of the three field components,
-// and their inverse transforms, keeping the outputs x < 128 (the mesh
-// planes the gather reads).  The unfused path's three whole spectra are
-// never written or read back.  256 = 16 x 16: a block of 256 threads takes
-// 16 columns, 16 threads a column, each thread 16 points in registers; a
-// transform is two 16-point DFTs with the 256-point twiddles between them
-// and one transpose through shared memory (rows of 17 against bank
-// conflicts; 273 float2 a column keeps the column-major staging
-// conflict-free too).
-constexpr int kXLen = 256;
-constexpr int kXCols = 16;
-constexpr int kXStride = 273;
+// Fused x pass of the single-precision mesh for a padded x length of 256 or
+// 128 (a 128- or 64-node mesh axis).  Per (ky, kz) column of the 2D-
+// transformed mesh planes: the forward transform along x (inputs of the upper
+// half are the zero padding), the products with i G_c of the three field
+// components, and their inverse transforms, keeping the lower half of the
+// outputs (the mesh planes the gather reads).  The unfused path's three whole
+// spectra are never written or read back, and its eight transform launches
+// and the product are one.  LEN = 16 T: T threads a column (16 or 8), each
+// thread 16 points in registers; a transform is 16-point DFTs and T-point
+// DFTs (one or two per thread) with the LEN-point twiddles between them and
+// one transpose through shared memory (rows of 17 against bank conflicts; an
+// odd column stride keeps the column-major staging conflict-free too).  Issue
+// bound on its butterflies: 76 us at 256 (33,024 columns; one template for
+// both lengths spilled there and took 84); 18 us at 128 (8,320 columns), where
+// the separate passes took 63.
+constexpr int kXThreads = 256;
+template <int LEN>
+struct XShape {
+    static constexpr int kT = LEN / 16;                   // threads a column, length of the second DFT
+    static constexpr uint32_t kCols = kXThreads / kT;     // columns a block
+    static constexpr int kStride = kT * 17 + 1;
+    static_assert(kStride % 2 == 1 && kStride > LEN / 2, "column stride");
+};
+inline bool xpass_fused(int m0) { return m0 == 256 || m0 == 128; }
 
 __device__ __forceinline__ float2 cmulf(float2 a, float2 b) {
     return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
@@ -447,27 +456,51 @@ __device__ __forceinline__ void dft16(float2 (&v)[16]) {
     for (int k = 0; k < 16; ++k) v[k] = t[k];
 }
 
+// 8-point DFT of v[0], v[S], ..., v[7 S] in place: n = 4 n1 + n2 as above with
+// n1 < 2: 2-point DFTs over n1, twiddles w8^(n2 k1), 4-point DFTs over n2.
+template <bool INV, int S>
+__device__ __forceinline__ void dft8(float2* v) {
+    constexpr float r2 = 0.707106781186547524f;
+    float2 e[4], o[4];
+#pragma unroll
+    for (int n2 = 0; n2 < 4; ++n2) {
+        const float2 a = v[n2 * S], b = v[(4 + n2) * S];
+        e[n2] = make_float2(a.x + b.x, a.y + b.y);
+        o[n2] = make_float2(a.x - b.x, a.y - b.y);
+    }
+    o[1] = cmulf(o[1], make_float2(r2, INV ? r2 : -r2));
+    o[2] = INV ? make_float2(-o[2].y, o[2].x) : make_float2(o[2].y, -o[2].x);
+    o[3] = cmulf(o[3], make_float2(-r2, INV ? r2 : -r2));
+    dft4<INV>(e[0], e[1], e[2], e[3]);
+    dft4<INV>(o[0], o[1], o[2], o[3]);
+#pragma unroll
+    for (int k2 = 0; k2 < 4; ++k2) {
+        v[2 * k2 * S] = e[k2];
+        v[(2 * k2 + 1) * S] = o[k2];
+    }
+}
+
 // in: the mesh planes x < 128 of the 2D-transformed charge, [x][ky][kz];
 // gf: the folded kernels, [c][ky][kz][kx] (k_sc_fold with kx_inner);
 // out: component c's planes x < 128 after the x pass, at c * 128 * P;
 // tw: exp(-2 pi i m / 256), m < 256.
-__global__ void __launch_bounds__(256, 3) k_sc_xconv(MeshGeom g, const float2* __restrict__ in,
-                                                  const float* __restrict__ gf, const float2* __restrict__ tw,
-                                                  float2* __restrict__ out) {
-    __shared__ float2 buf[kXCols * kXStride];
-    __shared__ float2 w[kXLen];
+__global__ void __launch_bounds__(256, 3) k_sc_xconv256(MeshGeom g, const float2* __restrict__ in,
+                                                        const float* __restrict__ gf,
+                                                        const float2* __restrict__ tw, float2* __restrict__ out) {
+    __shared__ float2 buf[XShape<256>::kCols * XShape<256>::kStride];
+    __shared__ float2 w[256];
     const FoldGeom f = fold_geom(g);
     const uint32_t P = static_cast<uint32_t>(g.m1) * static_cast<uint32_t>(f.hz);    // (ky, kz) columns
-    const uint32_t j0 = blockIdx.x * kXCols;
+    const uint32_t j0 = blockIdx.x * XShape<256>::kCols;
     const int col = threadIdx.x >> 4, t = threadIdx.x & 15;
     w[threadIdx.x] = tw[threadIdx.x];
-    for (int e = threadIdx.x; e < (kXLen / 2) * kXCols; e += blockDim.x) {
+    for (int e = threadIdx.x; e < 128 * 16; e += blockDim.x) {
         const int x = e >> 4, c = e & 15;
         const uint32_t j = j0 + c;
-        buf[c * kXStride + x] = j < P ? in[static_cast<size_t>(x) * P + j] : make_float2(0.f, 0.f);
+        buf[c * XShape<256>::kStride + x] = j < P ? in[static_cast<size_t>(x) * P + j] : make_float2(0.f, 0.f);
     }
     __syncthreads();
-    float2* bc = buf + col * kXStride;
+    float2* bc = buf + col * XShape<256>::kStride;
     float2 v[16];
     // forward: x = 16 x1 + t, k = k1 + 16 k2
 #pragma unroll
@@ -494,9 +527,9 @@ __global__ void __launch_bounds__(256, 3) k_sc_xconv(MeshGeom g, const float2* _
 #pragma unroll
         for (int k2 = 0; k2 < 16; ++k2) {
             const int kx = t + 16 * k2;
-            const int kxf = min(kx, kXLen - kx);
+            const int kxf = min(kx, 256 - kx);
             float G = live ? gc[kxf] : 0.f;
-            if (c == 0 && kx > kXLen / 2) G = -G;
+            if (c == 0 && kx > 256 / 2) G = -G;
             if (c == 1) G *= sy;
             v[k2] = make_float2(-G * X[k2].y, G * X[k2].x);
         }
@@ -516,10 +549,98 @@ __global__ void __launch_bounds__(256, 3) k_sc_xconv(MeshGeom g, const float2* _
 #pragma unroll
         for (int q = 0; q < 8; ++q) bc[t + 16 * q] = v[q];
         __syncthreads();
-        float2* oc = out + static_cast<size_t>(c) * (kXLen / 2) * P;
-        for (int e = threadIdx.x; e < (kXLen / 2) * kXCols; e += blockDim.x) {
+        float2* oc = out + static_cast<size_t>(c) * (256 / 2) * P;
+        for (int e = threadIdx.x; e < 128 * 16; e += blockDim.x) {
             const int x = e >> 4, cc = e & 15;
-            if (j0 + cc < P) oc[static_cast<size_t>(x) * P + j0 + cc] = buf[cc * kXStride + x];
+            if (j0 + cc < P) oc[static_cast<size_t>(x) * P + j0 + cc] = buf[cc * XShape<256>::kStride + x];
+        }
+    }
+}
+
+// The same for LEN = 128 = 16 T (T = 8): two second DFTs a thread.
+// Forward: x = T x1 + t, kx = k1 + 16 k2: 16-point DFTs over x1 (thread t),
+// twiddles w^(t k1), T-point DFTs over t for each k1.  Thread t holds k1 =
+// t + T j, j < 16 / T, and of each k2 < T, in register P j + ... below:
+// v[k2 * (16 / T) + j].  Inverse: x = r + T q: T-point DFTs over k2 for each
+// k1, twiddles, 16-point DFTs over k1 (thread r); q < 8 is kept.
+__global__ void __launch_bounds__(kXThreads, 3) k_sc_xconv128(MeshGeom g, const float2* __restrict__ in,
+                                                              const float* __restrict__ gf,
+                                                              const float2* __restrict__ tw,
+                                                              float2* __restrict__ out) {
+    constexpr int LEN = 128;
+    using X = XShape<LEN>;
+    constexpr int T = X::kT, J = 16 / T;
+    constexpr uint32_t kHalf = LEN / 2;
+    __shared__ float2 buf[X::kCols * X::kStride];
+    __shared__ float2 w[LEN];
+    const FoldGeom f = fold_geom(g);
+    const uint32_t P = static_cast<uint32_t>(g.m1) * static_cast<uint32_t>(f.hz);    // (ky, kz) columns
+    const uint32_t j0 = blockIdx.x * X::kCols;
+    const int col = static_cast<int>(threadIdx.x / T), t = static_cast<int>(threadIdx.x % T);
+    if (threadIdx.x < LEN) w[threadIdx.x] = tw[threadIdx.x];
+    for (uint32_t e = threadIdx.x; e < kHalf * X::kCols; e += kXThreads) {
+        const uint32_t x = e / X::kCols, c = e % X::kCols;
+        const uint32_t j = j0 + c;
+        buf[c * X::kStride + x] = j < P ? in[static_cast<size_t>(x) * P + j] : make_float2(0.f, 0.f);
+    }
+    __syncthreads();
+    float2* bc = buf + col * X::kStride;
+    float2 v[16];
+#pragma unroll
+    for (int x1 = 0; x1 < 16; ++x1) v[x1] = x1 < 8 ? bc[T * x1 + t] : make_float2(0.f, 0.f);
+    __syncthreads();
+    dft16<false>(v);
+#pragma unroll
+    for (int k1 = 0; k1 < 16; ++k1) bc[t * 17 + k1] = cmulf(v[k1], w[(t * k1) & (LEN - 1)]);
+    __syncthreads();
+#pragma unroll
+    for (int x2 = 0; x2 < T; ++x2) {
+#pragma unroll
+        for (int j = 0; j < J; ++j) v[x2 * J + j] = bc[x2 * 17 + t + T * j];
+    }
+    dft8<false, J>(v);
+    dft8<false, J>(v + 1);
+    float2 Xk[16];                                  // Xk[k2 J + j] = spectrum at kx = t + T j + 16 k2
+#pragma unroll
+    for (int k = 0; k < 16; ++k) Xk[k] = v[k];
+    const uint32_t j = j0 + col;
+    const bool live = j < P;
+    const int ky = live ? static_cast<int>(j / f.hz) : 0, kz = live ? static_cast<int>(j % f.hz) : 0;
+    const int kyf = min(ky, g.m1 - ky);
+    const float sy = 2 * ky > g.m1 ? -1.f : 1.f;
+    for (int c = 0; c < 3; ++c) {
+        // kernel values in [ky][kz][kx] order: a column's kx run is contiguous
+        const float* gc = gf + c * f.n + (static_cast<size_t>(kyf) * f.hz + kz) * f.hx;
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+            const int kx = t + T * (k % J) + 16 * (k / J);
+            const int kxf = min(kx, LEN - kx);
+            float G = live ? gc[kxf] : 0.f;
+            if (c == 0 && kx > static_cast<int>(kHalf)) G = -G;
+            if (c == 1) G *= sy;
+            v[k] = make_float2(-G * Xk[k].y, G * Xk[k].x);
+        }
+        dft8<true, J>(v);
+        dft8<true, J>(v + 1);                       // v[r J + j]: k1 = t + T j, r < T
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+            const int r = k / J, k1 = t + T * (k % J);
+            const float2 wr = w[(r * k1) & (LEN - 1)];
+            bc[r * 17 + k1] = cmulf(v[k], make_float2(wr.x, -wr.y));
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k1 = 0; k1 < 16; ++k1) v[k1] = bc[t * 17 + k1];
+        dft16<true>(v);
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < 8; ++q) bc[t + T * q] = v[q];
+        __syncthreads();
+        float2* oc = out + static_cast<size_t>(c) * kHalf * P;
+        for (uint32_t e = threadIdx.x; e < kHalf * X::kCols; e += kXThreads) {
+            const uint32_t x = e / X::kCols, cc = e % X::kCols;
+            if (j0 + cc < P) oc[static_cast<size_t>(x) * P + j0 + cc] = buf[cc * X::kStride + x];
         }
     }
 }
@@ -1016,10 +1137,10 @@ struct SpaceChargeSolver {
     float* gfold_f = nullptr;             // three folded kernels, one block
     cufftHandle xpass = 0, inv2 = 0;
     bool have_xpass = false, have_inv2 = false;
-    // a padded x length of 256 runs the fused x pass (k_sc_xconv) in place
-    // of the cuFFT x passes and the separate kernel products
+    // a padded x length of 256 or 128 runs the fused x pass (k_sc_xconv) in
+    // place of the cuFFT x passes and the separate kernel products
     bool xfused = false;
-    float2* tw256 = nullptr;
+    float2* xtw = nullptr;
     // other devices' ions in this solve (icb_spacecharge_set_peers); cap
     // covers own_cap own ions plus the peers
     uint32_t own_cap = 0;
@@ -1046,7 +1167,7 @@ struct SpaceChargeSolver {
             if (p) cudaFree(p);
         if (egrid[0]) cudaFree(egrid[0]);   // one block holds the three grids
         for (void* q : {static_cast<void*>(rho_f), static_cast<void*>(rho_hat_f), static_cast<void*>(tmp_hat_f),
-                        static_cast<void*>(egrid_f), static_cast<void*>(gfold_f), static_cast<void*>(tw256)})
+                        static_cast<void*>(egrid_f), static_cast<void*>(gfold_f), static_cast<void*>(xtw)})
             if (q) cudaFree(q);
         for (int c = 0; c < 3; ++c) {
             if (ghat[c]) cudaFree(ghat[c]);
@@ -1213,7 +1334,7 @@ int sc_create(const icb_spacecharge_config& c, uint64_t n_ions, bool pp_float, c
             SC_CUDA(cudaGetLastError());
             if (f32) {
                 const size_t nf = fold_geom(g).n;
-                k_sc_fold<<<blocks_for(nf, 256), 256, 0, s>>>(g, gh, g.m0 == kXLen ? 1 : 0, S.gfold_f + a * nf);
+                k_sc_fold<<<blocks_for(nf, 256), 256, 0, s>>>(g, gh, xpass_fused(g.m0) ? 1 : 0, S.gfold_f + a * nf);
                 SC_CUDA(cudaGetLastError());
             }
         }
@@ -1240,14 +1361,14 @@ int sc_create(const icb_spacecharge_config& c, uint64_t n_ions, bool pp_float, c
             SC_FFT(cufftPlanMany(&S.fwd, 2, n2d, nullptr, 1, 0, nullptr, 1, 0, CUFFT_R2C, g.n0));
             S.have_fwd = true;
             SC_FFT(cufftSetStream(S.fwd, s));
-            S.xfused = g.m0 == kXLen;
+            S.xfused = xpass_fused(g.m0);
             if (S.xfused) {
-                std::vector<float2> tw(kXLen);
-                for (int m = 0; m < kXLen; ++m)
-                    tw[m] = make_float2(static_cast<float>(std::cos(2.0 * kPi * m / kXLen)),
-                                        static_cast<float>(-std::sin(2.0 * kPi * m / kXLen)));
-                SC_CUDA(dev_alloc(&S.tw256, kXLen));
-                SC_CUDA(cudaMemcpy(S.tw256, tw.data(), kXLen * sizeof(float2), cudaMemcpyHostToDevice));
+                std::vector<float2> tw(static_cast<size_t>(g.m0));
+                for (int m = 0; m < g.m0; ++m)
+                    tw[m] = make_float2(static_cast<float>(std::cos(2.0 * kPi * m / g.m0)),
+                                        static_cast<float>(-std::sin(2.0 * kPi * m / g.m0)));
+                SC_CUDA(dev_alloc(&S.xtw, tw.size()));
+                SC_CUDA(cudaMemcpy(S.xtw, tw.data(), tw.size() * sizeof(float2), cudaMemcpyHostToDevice));
             } else {
                 int n1d[1] = {g.m0};
                 const int cols = g.m1 * (g.m2 / 2 + 1);
@@ -1388,7 +1509,12 @@ int sc_solve(SpaceChargeSolver* S, const double* x, const double* y, const doubl
         SC_FFT(cufftExecR2C(S->fwd, S->rho_f, S->rho_hat_f));
         if (S->xfused) {
             const size_t P = static_cast<size_t>(g.m1) * (g.m2 / 2 + 1);
-            k_sc_xconv<<<blocks_for(P, kXCols), 256, 0, s>>>(g, S->rho_hat_f, S->gfold_f, S->tw256, S->tmp_hat_f);
+            if (g.m0 == 256)
+                k_sc_xconv256<<<blocks_for(P, XShape<256>::kCols), kXThreads, 0, s>>>(g, S->rho_hat_f, S->gfold_f,
+                                                                                        S->xtw, S->tmp_hat_f);
+            else
+                k_sc_xconv128<<<blocks_for(P, XShape<128>::kCols), kXThreads, 0, s>>>(g, S->rho_hat_f, S->gfold_f,
+                                                                                        S->xtw, S->tmp_hat_f);
             SC_CUDA(cudaGetLastError());
             SC_FFT(cufftExecC2R(S->inv2, S->tmp_hat_f, S->egrid_f));
         } else {
