@@ -15,6 +15,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <numeric>
 #include <random>
 #include <string>
@@ -472,6 +473,39 @@ struct DevVec {
 
 }  // namespace
 
+// Pool for the memory of one-shot calls.  cudaMalloc and cudaFree of a call's
+// workspace cost 0.6 ms on the host, more than half of a short training run;
+// the pool hands the same memory to the next call in a few microseconds.  It
+// keeps at most kCallPoolKeep bytes per device between calls (the driver
+// releases the rest when a call's stream is synchronised), belongs to no
+// handle, and is safe with several threads and streams: allocations are
+// stream ordered and the driver orders their reuse.  Null when the device
+// has no pools or the creation fails (the caller then allocates plainly).
+constexpr uint64_t kCallPoolKeep = 32ull << 20;
+static cudaMemPool_t call_pool(int device) {
+    static std::mutex m;
+    static cudaMemPool_t pools[64] = {};
+    if (device < 0 || device >= 64) return nullptr;
+    std::lock_guard<std::mutex> lock(m);
+    uint64_t keep = kCallPoolKeep;
+    // (setting the threshold also finds out whether a device reset took the pool)
+    if (pools[device] && cudaMemPoolSetAttribute(pools[device], cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess)
+        return pools[device];
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    cudaMemPool_t pool = nullptr;
+    if (cudaMemPoolCreate(&pool, &props) != cudaSuccess ||
+        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+        cudaGetLastError();
+        if (pool) cudaMemPoolDestroy(pool);
+        return nullptr;
+    }
+    pools[device] = pool;
+    return pool;
+}
+
 // Collision-path parameter blocks: B fragments of W2 (BF16 pairs) and the
 // float block (W1, W3 rounded to BF16; biases FP32).
 void mlp_pack(const float* params, std::vector<uint32_t>& frag, std::vector<float>& fblock) {
@@ -556,16 +590,41 @@ int icb_mlp_init(uint64_t seed, float* params) {
     return ICB_OK;
 }
 
+// Memory of one training or gradient call from the library's pool of the
+// device (call_pool), stream ordered; plain device memory where there is none.
+struct CallMem {
+    unsigned char* p = nullptr;
+    cudaStream_t s = nullptr;
+    bool pooled = false;
+    ~CallMem() {
+        if (!p) return;
+        if (pooled) cudaFreeAsync(p, s);
+        else cudaFree(p);
+    }
+    cudaError_t alloc(size_t bytes, int device, cudaStream_t stream) {
+        s = stream;
+        if (cudaMemPool_t pool = call_pool(device)) {
+            if (cudaMallocFromPoolAsync(reinterpret_cast<void**>(&p), bytes, pool, s) == cudaSuccess) {
+                pooled = true;
+                return cudaSuccess;
+            }
+            cudaGetLastError();
+            p = nullptr;
+        }
+        return cudaMalloc(reinterpret_cast<void**>(&p), bytes);
+    }
+};
+
 // Device workspace of one training or gradient call, one allocation: the
 // samples, the parameter state, the permutation and the rows of one chunk.
 struct MlpWork {
-    DevVec<unsigned char> mem;
+    CallMem mem;
     float *x = nullptr, *y = nullptr, *params = nullptr, *m = nullptr, *v = nullptr, *gsum = nullptr, *rows = nullptr,
           *cols = nullptr;
     uint32_t* perm = nullptr;
     double *lsum = nullptr, *loss = nullptr;
     uint32_t ld = 0;
-    cudaError_t alloc(uint64_t n, uint64_t batch, bool with_perm) {
+    cudaError_t alloc(uint64_t n, uint64_t batch, bool with_perm, int device, cudaStream_t stream) {
         const uint64_t chunk = std::min<uint64_t>(batch, kChunk);
         ld = static_cast<uint32_t>((chunk + kGroup - 1) / kGroup * kGroup);
         size_t at = 0;
@@ -577,7 +636,7 @@ struct MlpWork {
         const size_t ocol = take(static_cast<size_t>(kCols) * ld * sizeof(float));
         const size_t operm = take(with_perm ? n * sizeof(uint32_t) : 0);
         const size_t ol = take(2 * sizeof(double));
-        const cudaError_t e = mem.alloc(at);
+        const cudaError_t e = mem.alloc(at, device, stream);
         if (e != cudaSuccess) return e;
         x = reinterpret_cast<float*>(mem.p + ox);
         y = reinterpret_cast<float*>(mem.p + oy);
@@ -658,7 +717,7 @@ int icb_mlp_train(int device, const icb_mlp_train_config* cfg, uint64_t n, const
     const uint32_t B = static_cast<uint32_t>(cfg->batch);
     const bool bf16 = cfg->bf16_forward != 0;
     MlpWork w;
-    MLP_CUDA(w.alloc(n, B, true));
+    MLP_CUDA(w.alloc(n, B, true, device, s));
     MLP_CUDA(batch_attrs(bf16, true));
     MLP_CUDA(cudaMemcpyAsync(w.x, x, 2 * n * sizeof(float), cudaMemcpyHostToDevice, s));
     MLP_CUDA(cudaMemcpyAsync(w.y, y, n * sizeof(float), cudaMemcpyHostToDevice, s));
@@ -742,16 +801,15 @@ int icb_mlp_gradients(int device, const float* params, uint64_t n, const float* 
     if (n == 0 || n > (1u << 20)) return set_error(ICB_ERR_INVALID_ARGUMENT, "need 1 <= n <= 2^20");
     MLP_CUDA(cudaSetDevice(device));
     MlpWork w;
-    DevVec<float> dg;
-    MLP_CUDA(w.alloc(n, n, false));
-    MLP_CUDA(dg.alloc(kMlpParams));
+    MLP_CUDA(w.alloc(n, n, false, device, nullptr));
+    float* const dg = w.m;           // no Adam state in this call
     MLP_CUDA(batch_attrs(false, false));
     MLP_CUDA(cudaMemcpy(w.x, x, 2 * n * sizeof(float), cudaMemcpyHostToDevice));
     MLP_CUDA(cudaMemcpy(w.y, y, n * sizeof(float), cudaMemcpyHostToDevice));
     MLP_CUDA(cudaMemcpy(w.params, params, kMlpParams * sizeof(float), cudaMemcpyHostToDevice));
     MLP_CUDA(cudaMemset(w.loss, 0, sizeof(double)));
-    if (int r = launch_batch(false, false, w, 0, n, AdamState{}, dg.p, nullptr)) return r;
-    MLP_CUDA(cudaMemcpy(grad, dg.p, kMlpParams * sizeof(float), cudaMemcpyDeviceToHost));
+    if (int r = launch_batch(false, false, w, 0, n, AdamState{}, dg, nullptr)) return r;
+    MLP_CUDA(cudaMemcpy(grad, dg, kMlpParams * sizeof(float), cudaMemcpyDeviceToHost));
     double l = 0.0;
     MLP_CUDA(cudaMemcpy(&l, w.loss, sizeof(double), cudaMemcpyDeviceToHost));
     if (loss) *loss = l / static_cast<double>(n);
