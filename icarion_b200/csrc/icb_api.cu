@@ -115,10 +115,6 @@ __global__ void k_to_hilo(const double* __restrict__ src, float* __restrict__ hi
         lo[i] = static_cast<float>(src[i] - static_cast<double>(h));
     }
 }
-__global__ void k_from_float(const float* __restrict__ src, double* __restrict__ dst, uint64_t n) {
-    const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i < n) dst[i] = static_cast<double>(src[i]);
-}
 __global__ void k_from_hilo(const float* __restrict__ hi, const float* __restrict__ lo, double* __restrict__ dst, uint64_t n) {
     const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i < n) dst[i] = static_cast<double>(hi[i]) + static_cast<double>(lo[i]);
@@ -142,14 +138,12 @@ __global__ void k_flags_update(const uint8_t* __restrict__ active, uint8_t* __re
     if ((f & kFlagBorn) != 0) f = active[i] ? static_cast<uint8_t>(f | kFlagActive) : static_cast<uint8_t>(f & ~kFlagActive);
     flags[i] = f;
 }
-__global__ void k_flags_out(const uint8_t* __restrict__ flags, uint8_t* __restrict__ active, uint64_t n) {
-    const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i < n) active[i] = (flags[i] & kFlagActive) ? 1 : 0;
-}
-// One ion chunk of the overlapped host path, in one launch each way: the
-// staged double velocities (three arrays `stride` apart) to float when vx is
-// given, and the host activity bytes into the flags (k_to_float x 3 +
-// k_flags_update); and back (k_from_float x 3 + k_flags_out).
+// The state of an ion chunk (or of all ions) between host and working form,
+// in one launch each way: the staged double velocities (three arrays `stride`
+// apart) to float when vx is given, and the host activity bytes into the
+// flags (k_to_float x 3 + k_flags_update); and back.  One launch per array
+// with a staging array of one, which waits for each array's copy before the
+// next conversion, cost a download 30-40 us.
 __global__ void k_chunk_in(const double* __restrict__ stage, uint64_t stride, float* __restrict__ vx,
                            float* __restrict__ vy, float* __restrict__ vz, const uint8_t* __restrict__ active,
                            uint8_t* __restrict__ flags, uint64_t n) {
@@ -351,11 +345,10 @@ struct icb_handle {
     DevBuf<double> ehss_rgas;
     bool mlp_ready = false;
     // host fast path: copy and copy-back streams, per-chunk compute streams
-    // and events, velocity staging (3n)
+    // and events
     cudaStream_t copy_stream = nullptr, copy_back_stream = nullptr;
     std::vector<cudaStream_t> chunk_streams;
     std::vector<cudaEvent_t> hev;
-    DevBuf<double> hstage;
     // space charge (solved before every step when configured)
     SpaceChargeSolver* sc = nullptr;
     double sc_emax_base = 0.0;         // ensemble 0's field bound without space charge
@@ -852,7 +845,8 @@ int enqueue_tf_tables(icb_handle* h, uint32_t K, cudaStream_t st) {
 // a time-dependent field are built first unless the caller built them
 // (build_tf = false).
 int launch_step(icb_handle* h, uint32_t K, int do_push, int do_collide, int do_finalize, uint64_t lo = 0,
-                uint64_t hi = ~0ull, cudaStream_t stream = nullptr, bool build_tf = true) {
+                uint64_t hi = ~0ull, cudaStream_t stream = nullptr, bool build_tf = true,
+                bool advance_clock = false) {
     cudaStream_t st = stream ? stream : h->stream;
     if (build_tf) {
         if (int r = enqueue_tf_tables(h, K, st)) return r;
@@ -959,6 +953,14 @@ int launch_step(icb_handle* h, uint32_t K, int do_push, int do_collide, int do_f
                     E.sp_fAmean = static_cast<float>(E.A * E.mean_th);
                 }
             }
+            // the launch's last CTA advances the engine clock (no launch for it)
+            if (e0 + ne == n_ens && lo == 0 && hi >= h->n && advance_clock) {
+                p.clk_step = h->step_dev.p;
+                p.clk_t = h->t_dev.p;
+                p.clk_dt = h->dt_dev.p;
+                p.clk_ens = static_cast<uint32_t>(n_ens);
+                p.clk_ticket = h->counters.p + kCntTicket;
+            }
             cudaError_t err1;
             switch (h->cfg.precision) {
                 case ICB_PREC_FP64: err1 = launch_step1_fp64(h->coll, p, st); break;
@@ -1018,10 +1020,17 @@ int enqueue_advance(icb_handle* h, uint64_t n_steps, size_t n_timed) {
             if (timed) ++h->sc_timed;
         }
         if (j < n_timed) ICB_CUDA(cudaEventRecord(h->kev[2 * j], s));
-        if (int r = launch_step(h, K, 1, 1, 1)) return r;
+        // the per-step kernel advances the clock itself when its last chunk of
+        // ensembles has ions
+        const bool own_clock = h->cfg.collision_test == ICB_TEST_PER_STEP &&
+                               h->ens_off[static_cast<size_t>(ne)] >
+                                   h->ens_off[static_cast<size_t>((ne - 1) / kMaxLaunchEns * kMaxLaunchEns)];
+        if (int r = launch_step(h, K, 1, 1, 1, 0, ~0ull, nullptr, true, own_clock)) return r;
         if (j < n_timed) ICB_CUDA(cudaEventRecord(h->kev[2 * j + 1], s));
-        ICB_CUDA(launch_clock_advance(h->step_dev.p, h->t_dev.p, h->dt_dev.p, ne, K, s));
-        ++h->launches;
+        if (!own_clock) {
+            ICB_CUDA(launch_clock_advance(h->step_dev.p, h->t_dev.p, h->dt_dev.p, ne, K, s));
+            ++h->launches;
+        }
         left -= K;
         ++j;
     }
@@ -1332,7 +1341,7 @@ int icb_upload_ions(icb_handle* h, uint64_t n,
         ICB_CUDA(h->t_death.alloc(n)); ICB_CUDA(h->t_arr.alloc(n)); ICB_CUDA(h->birth.alloc(n));
         ICB_CUDA(h->zprev.alloc(n));
         ICB_CUDA(h->flags.alloc(n)); ICB_CUDA(h->active_stage.alloc(n));
-        ICB_CUDA(h->stage.alloc(f64 ? 0 : n));
+        ICB_CUDA(h->stage.alloc(f64 ? 0 : 3 * n));   // a third per axis
         h->n = n;
     }
     h->first_id = first_ion_id;
@@ -1467,10 +1476,12 @@ int icb_download_ions(icb_handle* h, double* x, double* y, double* z,
     for (int a = 0; a < 3; ++a) {
         if (!pos[a]) continue;
         if (h->hilo()) {
-            k_from_hilo<<<g, 256, 0, s>>>(ph[a]->p, pl[a]->p, h->stage.p, n);
+            // (its own third of the staging; the velocities' conversion follows
+            // these copies on the stream)
+            double* st = h->stage.p + static_cast<size_t>(a) * n;
+            k_from_hilo<<<g, 256, 0, s>>>(ph[a]->p, pl[a]->p, st, n);
             ICB_CUDA(cudaGetLastError());
-            ICB_CUDA(cudaMemcpyAsync(pos[a], h->stage.p, bytes, cudaMemcpyDeviceToHost, s));
-            ICB_CUDA(cudaStreamSynchronize(s));
+            ICB_CUDA(cudaMemcpyAsync(pos[a], st, bytes, cudaMemcpyDeviceToHost, s));
         } else {
             ICB_CUDA(cudaMemcpyAsync(pos[a], pd[a]->p, bytes, cudaMemcpyDeviceToHost, s));
         }
@@ -1478,22 +1489,19 @@ int icb_download_ions(icb_handle* h, double* x, double* y, double* z,
     double* vel[3] = {vx, vy, vz};
     DevBuf<double>* vd[3] = {&h->vxd, &h->vyd, &h->vzd};
     DevBuf<float>* vf[3] = {&h->vxf, &h->vyf, &h->vzf};
+    // velocities and activity bytes: one conversion launch, then the copies
+    const bool conv = !h->fp64() && (vel[0] || vel[1] || vel[2]);
+    if (conv || active) {
+        k_chunk_out<<<g, 256, 0, s>>>(conv ? vf[0]->p : nullptr, vf[1]->p, vf[2]->p, h->stage.p, n, h->flags.p,
+                                      h->active_stage.p, n);
+        ICB_CUDA(cudaGetLastError());
+    }
     for (int a = 0; a < 3; ++a) {
         if (!vel[a]) continue;
-        if (h->fp64()) {
-            ICB_CUDA(cudaMemcpyAsync(vel[a], vd[a]->p, bytes, cudaMemcpyDeviceToHost, s));
-        } else {
-            k_from_float<<<g, 256, 0, s>>>(vf[a]->p, h->stage.p, n);
-            ICB_CUDA(cudaGetLastError());
-            ICB_CUDA(cudaMemcpyAsync(vel[a], h->stage.p, bytes, cudaMemcpyDeviceToHost, s));
-            ICB_CUDA(cudaStreamSynchronize(s));
-        }
+        const double* src = h->fp64() ? vd[a]->p : h->stage.p + static_cast<size_t>(a) * n;
+        ICB_CUDA(cudaMemcpyAsync(vel[a], src, bytes, cudaMemcpyDeviceToHost, s));
     }
-    if (active) {
-        k_flags_out<<<g, 256, 0, s>>>(h->flags.p, h->active_stage.p, n);
-        ICB_CUDA(cudaGetLastError());
-        ICB_CUDA(cudaMemcpyAsync(active, h->active_stage.p, n, cudaMemcpyDeviceToHost, s));
-    }
+    if (active) ICB_CUDA(cudaMemcpyAsync(active, h->active_stage.p, n, cudaMemcpyDeviceToHost, s));
     if (death_time_s) ICB_CUDA(cudaMemcpyAsync(death_time_s, h->t_death.p, bytes, cudaMemcpyDeviceToHost, s));
     if (arrival_time_s) ICB_CUDA(cudaMemcpyAsync(arrival_time_s, h->t_arr.p, bytes, cudaMemcpyDeviceToHost, s));
     ICB_CUDA(cudaStreamSynchronize(s));
@@ -1945,7 +1953,6 @@ int icb_advance_host(icb_handle* h, uint64_t n_steps, int n_chunks, double* x, d
         ICB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         h->hev.push_back(e);
     }
-    if (!f64 && h->hstage.n < 3 * n) ICB_CUDA(h->hstage.alloc(3 * n));
     cudaStream_t s = h->stream, cs = h->copy_stream, bs = h->copy_back_stream;
     double* pos[3] = {x, y, z};
     double* vel[3] = {vx, vy, vz};
@@ -1974,7 +1981,7 @@ int icb_advance_host(icb_handle* h, uint64_t n_steps, int n_chunks, double* x, d
         if (cnt == 0) continue;
         for (int k = 0; k < 3; ++k) {
             ICB_CUDA(cudaMemcpyAsync(pd[k] + a, pos[k] + a, cnt * sizeof(double), cudaMemcpyHostToDevice, cs));
-            double* dst = f64 ? vd[k] + a : h->hstage.p + k * n + a;
+            double* dst = f64 ? vd[k] + a : h->stage.p + k * n + a;
             ICB_CUDA(cudaMemcpyAsync(dst, vel[k] + a, cnt * sizeof(double), cudaMemcpyHostToDevice, cs));
         }
         ICB_CUDA(cudaMemcpyAsync(h->active_stage.p + a, active + a, cnt, cudaMemcpyHostToDevice, cs));
@@ -1982,7 +1989,7 @@ int icb_advance_host(icb_handle* h, uint64_t n_steps, int n_chunks, double* x, d
         const unsigned g = grid_for(cnt, 256);
         cudaStream_t ks = h->chunk_streams[static_cast<size_t>(c)];
         ICB_CUDA(cudaStreamWaitEvent(ks, h->hev[2 * c], 0));
-        double* stage = f64 ? nullptr : h->hstage.p + a;
+        double* stage = f64 ? nullptr : h->stage.p + a;
         k_chunk_in<<<g, 256, 0, ks>>>(stage, n, f64 ? nullptr : vf[0] + a, f64 ? nullptr : vf[1] + a,
                                       f64 ? nullptr : vf[2] + a, h->active_stage.p + a, h->flags.p + a, cnt);
         ICB_CUDA(cudaGetLastError());
@@ -1995,7 +2002,7 @@ int icb_advance_host(icb_handle* h, uint64_t n_steps, int n_chunks, double* x, d
         ICB_CUDA(cudaStreamWaitEvent(bs, h->hev[2 * c + 1], 0));
         for (int k = 0; k < 3; ++k) {
             ICB_CUDA(cudaMemcpyAsync(pos[k] + a, pd[k] + a, cnt * sizeof(double), cudaMemcpyDeviceToHost, bs));
-            const double* src = f64 ? vd[k] + a : h->hstage.p + k * n + a;
+            const double* src = f64 ? vd[k] + a : h->stage.p + k * n + a;
             ICB_CUDA(cudaMemcpyAsync(vel[k] + a, src, cnt * sizeof(double), cudaMemcpyDeviceToHost, bs));
         }
         ICB_CUDA(cudaMemcpyAsync(active + a, h->active_stage.p + a, cnt, cudaMemcpyDeviceToHost, bs));
@@ -2020,8 +2027,12 @@ static int single_part(icb_handle* h, int push, int collide, int finalize, icb_r
         return fail(ICB_ERR_INVALID_ARGUMENT, "runs are limited to 2^31 engine steps");
     if (finalize) h->host_step += 1;
     cudaStream_t s = h->stream;
-    ICB_CUDA(cudaMemsetAsync(h->counters.p, 0, kNumCounters * sizeof(unsigned long long), s));
-    ICB_CUDA(cudaEventRecord(h->ev0, s));
+    // a call without statistics leaves the counters to the next one that
+    // reports (every such call zeroes them first) and needs no timing events
+    if (stats) {
+        ICB_CUDA(cudaMemsetAsync(h->counters.p, 0, kNumCounters * sizeof(unsigned long long), s));
+        ICB_CUDA(cudaEventRecord(h->ev0, s));
+    }
     h->launches = 0;
     h->sc_timed = 0;
     if (push && h->sc) {
@@ -2033,9 +2044,9 @@ static int single_part(icb_handle* h, int push, int collide, int finalize, icb_r
         ICB_CUDA(launch_clock_advance(h->step_dev.p, h->t_dev.p, h->dt_dev.p, ne, 1u, s));
         ++h->launches;
     }
+    if (!stats) return ICB_OK;
     ICB_CUDA(cudaEventRecord(h->ev1, s));
-    if (stats) return read_stats(h, stats, finalize ? 1 : 0, 0);
-    return ICB_OK;
+    return read_stats(h, stats, finalize ? 1 : 0, 0);
 }
 
 int icb_push(icb_handle* h) { return single_part(h, 1, 0, 0, nullptr); }

@@ -24,6 +24,7 @@ enum IntegKind : int { kBoris = 0, kRK4 = 1 };
 enum CounterSlot : int {
     kCntCandidates = 0, kCntCollisions = 1, kCntOverflow = 2, kCntDeaths = 3, kCntArrivals = 4,
     kCntStalls = 5,   // staged copies whose wait ran out (per-step kernel): an error
+    kCntTicket = 6,   // per-step kernel: CTAs done with the launch's clock (zero between launches)
     kNumCounters = 8
 };
 
@@ -197,6 +198,14 @@ struct StepParams {
     unsigned long long* counters;      // kNumCounters
     const unsigned long long* step_dev;// engine step index at launch start
     const double* t_dev;               // engine time per ensemble at launch start
+    // per-step kernel: the launch's last CTA advances the clock of clk_ens
+    // ensembles by n_steps (clk_step nullptr: it does not); clk_ticket counts
+    // the CTAs that are done with the old values
+    unsigned long long* clk_step;
+    double* clk_t;
+    const double* clk_dt;
+    unsigned long long* clk_ticket;
+    uint32_t clk_ens;
     uint64_t first_id;
     uint64_t seed;
     uint32_t rk[20];                   // Philox round keys of the seed

@@ -194,6 +194,33 @@ __device__ __forceinline__ int step1_ensemble(const StepParams& p, uint64_t i) {
     return lo;
 }
 
+// End of a CTA's work, reached by all its threads: the CTA that is last to be
+// done with the launch's clock advances it (step += n_steps, t_e += dt_e per
+// step, as k_clock_advance does), which spares each step a launch of 3 us and
+// the gap before it.  The ticket is one of the counters the host zeroes
+// before the call, and goes back to zero for the next launch.
+__device__ __forceinline__ void step1_advance_clock(const StepParams& p) {
+    if (p.clk_step == nullptr) return;
+    __shared__ int last;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(p.clk_ticket, 1ull) == static_cast<unsigned long long>(gridDim.x) - 1ull;
+    }
+    __syncthreads();
+    if (!last) return;
+    for (uint32_t e = threadIdx.x; e < p.clk_ens; e += blockDim.x) {
+        double t = p.clk_t[e];
+        const double d = p.clk_dt[e];
+        for (uint32_t k = 0; k < p.n_steps; ++k) t = t + d;
+        p.clk_t[e] = t;
+    }
+    if (threadIdx.x == 0) {
+        *p.clk_step += p.n_steps;
+        *p.clk_ticket = 0ull;
+    }
+}
+
 template <int PREC, int COLL>
 __global__ void __launch_bounds__(kStep1Block, Step1Shape<PREC>::kMinBlocks) k_step1(const __grid_constant__ StepParams p) {
     using R = typename PrecT<PREC>::R;
@@ -409,8 +436,10 @@ __global__ void __launch_bounds__(kStep1Block, Step1Shape<PREC>::kMinBlocks) k_s
             for (int q = 0; q < kStep1Stages; ++q)
                 if (issued[q] != uses[q]) (void)mbar_wait_bounded(&bar[q], uses[q] & 1u);
         }
+        step1_advance_clock(p);
         return;
     }
+    step1_advance_clock(p);
     const unsigned long long s0 = warp_sum_u32(n_cand), s1 = warp_sum_u32(n_coll), s2 = warp_sum_u32(n_ovf);
     const unsigned long long s3 = warp_sum_u32(n_dead), s4 = warp_sum_u32(n_arr);
     if ((j & 31) == 0) {
@@ -686,6 +715,7 @@ __global__ void __launch_bounds__(kStep1WsThreads, Step1WsShape<PREC>::kMinBlock
             }
         }
     }
+    step1_advance_clock(p);
     __syncthreads();
     if (tid == 0 && *abortp) atomicAdd(&p.counters[kCntStalls], 1ull);
     const unsigned long long s0 = warp_sum_u32(n_cand), s1 = warp_sum_u32(n_coll), s2 = warp_sum_u32(n_ovf);

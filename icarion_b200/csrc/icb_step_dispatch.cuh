@@ -6,8 +6,33 @@
 
 namespace icb {
 
+// Whether the float RF / time-dependent kernel should run with room for 24
+// resident warps per SM (80 registers, some spilled) instead of 20 (96): when
+// the launch then takes enough fewer rounds of resident warps.  Every warp
+// runs the same number of steps, so a round that is nearly empty still costs
+// most of a round: 3,126 warps (the 100,001-ion trap on 148 SMs) are 1.06
+// rounds of 20 per SM, 0.88 of 24: 1205 -> 913 us a pass; 8,192 warps (TIMS,
+// 262,144 ions) are 3 rounds either way and slower with 24 (1679 -> 1764 us).
+inline bool more_warps(dim3 grid, dim3 block) {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1)
+        return false;
+    const uint64_t warps = static_cast<uint64_t>(grid.x) * (block.x / 32u);
+    const uint64_t a = 20ull * static_cast<uint64_t>(sms), b = 24ull * static_cast<uint64_t>(sms);
+    const uint64_t ra = (warps + a - 1) / a, rb = (warps + b - 1) / b;
+    // a round of 24 warps costs about 1.26 of a round of 20
+    return 126ull * rb < 100ull * ra;
+}
+
 template <int PREC, int INTEG, int COLL, int FIELD, bool MAG>
 cudaError_t launch_one(const StepParams& p, dim3 grid, dim3 block, cudaStream_t s) {
+    if constexpr (PREC != kPrecFP64 && FIELD == kFieldLinearRF) {
+        if (p.do_push && p.do_collide && p.do_finalize && more_warps(grid, block)) {
+            k_step<PREC, INTEG, COLL, FIELD, MAG, true, 6><<<grid, block, 0, s>>>(p);
+            return cudaGetLastError();
+        }
+    }
     if (p.do_push && p.do_collide && p.do_finalize)
         k_step<PREC, INTEG, COLL, FIELD, MAG, true><<<grid, block, 0, s>>>(p);
     else

@@ -821,6 +821,10 @@ __global__ void __launch_bounds__(256) k_clock_advance(unsigned long long* step,
                                                        uint32_t K) {
     const uint32_t e = blockIdx.x;
     if (e == 0 && threadIdx.x == 0) *step += K;
+    if (K == 1u) {
+        if (threadIdx.x == 0) t[e] = t[e] + dt[e];
+        return;
+    }
     const double end = clock_sequence(t[e], dt[e], K, [](uint32_t, double) {});
     if (threadIdx.x == 0) t[e] = end;
 }
@@ -1510,8 +1514,9 @@ struct KernelShape {
     static constexpr int kMinBlocks = PREC == kPrecFP64 ? 4 : (FIELD == kFieldLinearRF ? 5 : 6);
 };
 
-template <int PREC, int INTEG, int COLL, int FIELD, bool MAG, bool FUSED>
-__global__ void __launch_bounds__(128, KernelShape<PREC, COLL, FIELD>::kMinBlocks) k_step(const __grid_constant__ StepParams p) {
+template <int PREC, int INTEG, int COLL, int FIELD, bool MAG, bool FUSED,
+          int MIN_BLOCKS = KernelShape<PREC, COLL, FIELD>::kMinBlocks>
+__global__ void __launch_bounds__(128, MIN_BLOCKS) k_step(const __grid_constant__ StepParams p) {
     using R = typename PrecT<PREC>::R;
     using Pos = typename PosOf<PREC>::T;
     using Snap = typename Pos::Snap;
