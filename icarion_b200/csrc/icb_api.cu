@@ -336,6 +336,7 @@ struct icb_handle {
     const double2* cs_tab = nullptr;   // FP64 collisions: functions of the 16-bit draws
     DevBuf<double> tf_tab;             // per-step field scalars, one launch chunk at a time
     bool any_tf = false;
+    bool own_capture = false;          // icb_advance is capturing its own graph
     int base_field_kind = kFieldUniform;
     // EHSS geometry: host copies per ensemble and the device arrays
     std::vector<std::vector<double4>> ehss_host;
@@ -792,6 +793,19 @@ bool rf_tab(const icb_handle* h, uint32_t K) {
 }
 bool needs_tab(const icb_handle* h, uint32_t K) { return h->any_tf || rf_tab(h, K); }
 
+// needs_tab, but false for an RF-only handle on a stream that its caller is
+// capturing: the lanes then evaluate the cosines, so that a captured graph
+// holds no pointer to a table that a longer later launch replaces (the
+// handle's own graphs are dropped then).
+int use_tab(const icb_handle* h, uint32_t K, cudaStream_t st, bool& use) {
+    use = needs_tab(h, K);
+    if (!use || h->any_tf || h->own_capture) return ICB_OK;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    ICB_CUDA(cudaStreamIsCapturing(st, &cs));
+    use = cs == cudaStreamCaptureStatusNone;
+    return ICB_OK;
+}
+
 // Room for the per-step field tables of launches of up to K steps (all
 // ensembles, plus the time sequences); allocates outside stream capture only.
 int ensure_tf_tab(icb_handle* h, uint32_t K, cudaStream_t st) {
@@ -817,8 +831,10 @@ int ensure_tf_tab(icb_handle* h, uint32_t K, cudaStream_t st) {
 // The time-only field scalars of every step of a K-step launch for the
 // ensembles with a time-dependent field, built on `st` before the step
 // kernels read them (stage 0 at t_k; RK4 adds the half step).
-int enqueue_tf_tables(icb_handle* h, uint32_t K, cudaStream_t st) {
-    if (!needs_tab(h, K)) return ICB_OK;
+// `use` tells whether the launch has a table.
+int enqueue_tf_tables(icb_handle* h, uint32_t K, cudaStream_t st, bool& use) {
+    if (int r = use_tab(h, K, st, use)) return r;
+    if (!use) return ICB_OK;
     if (int r = ensure_tf_tab(h, K, st)) return r;
     const uint32_t stride = tf_stride(h);
     const int n_ens = static_cast<int>(h->ens.size());
@@ -841,15 +857,15 @@ int enqueue_tf_tables(icb_handle* h, uint32_t K, cudaStream_t st) {
     return ICB_OK;
 }
 
-// Step kernels for ions [lo, hi) (all ions by default); the field tables of
-// a time-dependent field are built first unless the caller built them
-// (build_tf = false).
+// Step kernels for ions [lo, hi) (all ions by default); the launch's field
+// table is built first unless the caller has done so and says with have_tab
+// whether there is one (build_tf = false).
 int launch_step(icb_handle* h, uint32_t K, int do_push, int do_collide, int do_finalize, uint64_t lo = 0,
                 uint64_t hi = ~0ull, cudaStream_t stream = nullptr, bool build_tf = true,
-                bool advance_clock = false) {
+                bool advance_clock = false, bool have_tab = false) {
     cudaStream_t st = stream ? stream : h->stream;
     if (build_tf) {
-        if (int r = enqueue_tf_tables(h, K, st)) return r;
+        if (int r = enqueue_tf_tables(h, K, st, have_tab)) return r;
     }
     const int n_ens = static_cast<int>(h->ens.size());
     if ((h->coll == kCollIPMTable || h->coll == kCollIPMMLP || h->coll == kCollIPMQuad) && h->ipm_nE == 0)
@@ -921,7 +937,7 @@ int launch_step(icb_handle* h, uint32_t K, int do_push, int do_collide, int do_f
             p.ens[e] = h->ens_const[static_cast<size_t>(e0 + e)];
             if (p.ens[e].flow) p.flows = 1u;
         }
-        if (needs_tab(h, K)) {
+        if (have_tab) {
             p.tf_tab = h->tf_tab.p;
             p.tf_stride = tf_stride(h);
             p.rf_tab = rf_tab(h, K) ? 1u : 0u;
@@ -1530,7 +1546,9 @@ int icb_advance(icb_handle* h, uint64_t n_steps, icb_run_stats* stats) {
             }
             ICB_CUDA(cudaStreamBeginCapture(h->own_stream, cudaStreamCaptureModeThreadLocal));
             h->stream = h->own_stream;
+            h->own_capture = true;
             int r = enqueue_advance(h, n_steps, 0);
+            h->own_capture = false;
             h->stream = s;
             cudaError_t ce = cudaStreamEndCapture(h->own_stream, &g);
             if (r != ICB_OK) { if (g) cudaGraphDestroy(g); return r; }
@@ -1975,7 +1993,8 @@ int icb_advance_host(icb_handle* h, uint64_t n_steps, int n_chunks, double* x, d
     // last blocks finish), results on the copy-back stream.  Queued in chunk
     // order, the first chunk's steps start as soon as its inputs are in.
     // one field table for all chunks, ahead of every chunk's steps
-    if (int r = enqueue_tf_tables(h, static_cast<uint32_t>(n_steps), cs)) return r;
+    bool have_tab = false;
+    if (int r = enqueue_tf_tables(h, static_cast<uint32_t>(n_steps), cs, have_tab)) return r;
     for (int c = 0; c < n_chunks; ++c) {
         const uint64_t a = lim[static_cast<size_t>(c)], b = lim[static_cast<size_t>(c) + 1], cnt = b - a;
         if (cnt == 0) continue;
@@ -1993,7 +2012,8 @@ int icb_advance_host(icb_handle* h, uint64_t n_steps, int n_chunks, double* x, d
         k_chunk_in<<<g, 256, 0, ks>>>(stage, n, f64 ? nullptr : vf[0] + a, f64 ? nullptr : vf[1] + a,
                                       f64 ? nullptr : vf[2] + a, h->active_stage.p + a, h->flags.p + a, cnt);
         ICB_CUDA(cudaGetLastError());
-        if (int r = launch_step(h, static_cast<uint32_t>(n_steps), 1, 1, 1, a, b, ks, false)) return r;
+        if (int r = launch_step(h, static_cast<uint32_t>(n_steps), 1, 1, 1, a, b, ks, false, false, have_tab))
+            return r;
         k_chunk_out<<<g, 256, 0, ks>>>(f64 ? nullptr : vf[0] + a, f64 ? nullptr : vf[1] + a, f64 ? nullptr : vf[2] + a,
                                        stage, n, h->flags.p + a, h->active_stage.p + a, cnt);
         ICB_CUDA(cudaGetLastError());
