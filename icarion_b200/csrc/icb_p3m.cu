@@ -162,14 +162,17 @@ __global__ void __launch_bounds__(kStartThreads) k_sc_cell_start(const uint32_t*
 // particle-particle loops then read contiguous memory.
 // A float copy (position relative to the mesh origin, Coulomb constant times
 // the charge) serves the particle-particle loop: per slot (x, y, z, kq) as
-// the FP64 loop's distance prefilter, or, for the float loop (`pairs`), per
-// slot pair k = s / 2 as two float4 {x0, x1, y0, y1}, {z0, z1, kq0, kq1}:
-// the packed (two-lane) FP32 instructions then take each pair's values as
-// loaded.
+// the FP64 loop's distance prefilter, or, for the float loop (`quads`), per
+// four slots 4k .. 4k + 3 the even two's and then the odd two's as two float4
+// each, {x0, x2, y0, y2}, {z0, z2, kq0, kq2}: a lane that owns one parity
+// loads what the packed (two-wide) FP32 instructions take.
+__device__ __forceinline__ uint32_t quad_slot(uint32_t s) {
+    return 16u * (s >> 2) + 8u * (s & 1u) + ((s >> 1) & 1u);
+}
 __global__ void k_sc_permute(MeshGeom g, const double* __restrict__ x, const double* __restrict__ y,
                              const double* __restrict__ z, const double* __restrict__ q,
                              const uint32_t* __restrict__ vals, uint32_t n, uint32_t n_own, PeerIons peers,
-                             int pairs, double4* __restrict__ ps, float4* __restrict__ pf) {
+                             int quads, double4* __restrict__ ps, float4* __restrict__ pf) {
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
     const uint32_t j = vals[s];
@@ -177,9 +180,12 @@ __global__ void k_sc_permute(MeshGeom g, const double* __restrict__ x, const dou
     ps[s] = v;
     const float fx = static_cast<float>(v.x - g.lo0), fy = static_cast<float>(v.y - g.lo1);
     const float fz = static_cast<float>(v.z - g.lo2), fq = static_cast<float>(kCoulomb * v.w);
-    if (pairs) {
-        float* b = reinterpret_cast<float*>(pf) + 8u * (s >> 1) + (s & 1u);
-        b[0] = fx; b[2] = fy; b[4] = fz; b[6] = fq;
+    if (quads) {
+        // an ion outside the mesh (not a number included) shares a quad with
+        // ions inside: kept finite, so that its masked pairs add zero
+        auto fin = [](float v) { return fminf(fmaxf(v, -1e18f), 1e18f); };
+        float* b = reinterpret_cast<float*>(pf) + quad_slot(s);
+        b[0] = fin(fx); b[2] = fin(fy); b[4] = fin(fz); b[6] = fq;
     } else {
         pf[s] = make_float4(fx, fy, fz, fq);
     }
@@ -876,19 +882,32 @@ __device__ __forceinline__ float rcp_hw(float x) {
 // interpolation of the float mesh field and the particle-particle correction
 // in float arithmetic on positions relative to the mesh origin.
 //
-// Four lanes per ion, eight consecutive sorted ions per warp.  Partners are
-// read as slot pairs (k_sc_permute) and evaluated two at a time on the packed
+// Two lanes per ion, consecutive sorted ions in a warp.  A lane owns one slot
+// parity and takes two partners at a time (k_sc_permute's quads) on the packed
 // FP32 pipe (fma/add/mul .f32x2).  Each (x, y) neighbour column contributes
 // the z cells that reach within r_c of the ion given the column's distance
-// (lower bounds, padded for rounding): the ion's four lanes set up four
-// columns at once, then walk each column's slot range together, lane j
-// taking every fourth slot pair.  Pairs outside the range or outside
-// (min_d, r_c) add exactly nothing (the ion itself is at distance 0).
-constexpr int kGatherBlock = 128;
-constexpr int kGatherLanes = 4;
+// (lower bounds, padded for rounding): an ion's lanes set up one column each,
+// then walk each column's slot range together.  Pairs outside the range or
+// outside (min_d, r_c) add exactly nothing (the ion itself is at distance 0),
+// so an ion's field is the sum of its even and of its odd partners, each a
+// chain in slot order, whatever else the warp holds.  More lanes per ion would
+// split those chains: beside a very close pair every addition rounds at that
+// pair's size, and the order of the sum then shows in the ion's path.
+//
+// Bound: instruction issue and the packed-FP32 pipe (DRAM under 1 %).  A
+// warp's column walk lasts as long as its longest lane's, so it serves 16
+// ions, not 32, and walks their own columns, not the union of the warp's.  The
+// whole solve, this walk against one warp-wide union of 32 ions' columns:
+// 262,144 ions on 128^3 700 against 847 us, on 64^3 2,449 against 3,686;
+// 40,009 ions on 64^3 272 against 468, 10,007 ions on 64^3 159 against 268.
+// Tried (262,144 ions on 128^3 / 64^3, us): one lane per ion with both
+// parities in a packed accumulator 763 / 3,020; four lanes 677 / 2,245, with
+// the order above lost; 6 blocks per SM 706 / 2,428, 8: 708 / 2,543, 10: 727 /
+// 2,666; the partner loop unrolled by two 720 / 2,516.
+constexpr int kGatherBlock = 128, kGatherLanes = 2;
 
 template <bool POLY>
-__global__ void __launch_bounds__(kGatherBlock, 8) k_sc_gather_f32(MeshGeom g, PPParams pp,
+__global__ void __launch_bounds__(kGatherBlock, 7) k_sc_gather_f32(MeshGeom g, PPParams pp,
                             const double4* __restrict__ ps, const float4* __restrict__ pf,
                             const uint32_t* __restrict__ keys, const uint32_t* __restrict__ vals,
                             const uint32_t* __restrict__ start, uint32_t n, const uint32_t* __restrict__ slots,
@@ -917,19 +936,22 @@ __global__ void __launch_bounds__(kGatherBlock, 8) k_sc_gather_f32(MeshGeom g, P
         const int ci = static_cast<int>(t / g.n1);
         float fxi = 0.f, fyi = 0.f, fzi = 0.f;
         if (act) {
-            // lane j: the two z corners of the cell's (x, y) edge j
             const double4 pi4 = ps[s];
             const double fx = (pi4.x - g.lo0) * g.ih0 - ci;
             const double fy = (pi4.y - g.lo1) * g.ih1 - cj;
             const double fz = (pi4.z - g.lo2) * g.ih2 - ck;
-            const int ox = static_cast<int>(jl >> 1), oy = static_cast<int>(jl & 1u);
-            const size_t node = (static_cast<size_t>(ci + ox) * g.m1 + static_cast<size_t>(cj + oy)) * g.m2 +
-                                static_cast<size_t>(ck);
-            const double w0 = cic_w<double>(ox, oy, 0, fx, fy, fz), w1 = cic_w<double>(ox, oy, 1, fx, fy, fz);
-            E[0] = w0 * static_cast<double>(gx[node]) + w1 * static_cast<double>(gx[node + 1]);
-            E[1] = w0 * static_cast<double>(gy[node]) + w1 * static_cast<double>(gy[node + 1]);
-            E[2] = w0 * static_cast<double>(gz[node]) + w1 * static_cast<double>(gz[node + 1]);
-            const float* b = reinterpret_cast<const float*>(pf) + 8u * (s >> 1) + (s & 1u);
+            // each lane the whole interpolation
+#pragma unroll
+            for (int o = 0; o < 8; ++o) {
+                const int ox = o & 1, oy = (o >> 1) & 1, oz = o >> 2;
+                const size_t node = (static_cast<size_t>(ci + ox) * g.m1 + static_cast<size_t>(cj + oy)) * g.m2 +
+                                    static_cast<size_t>(ck + oz);
+                const double w = cic_w<double>(ox, oy, oz, fx, fy, fz);
+                E[0] += w * static_cast<double>(gx[node]);
+                E[1] += w * static_cast<double>(gy[node]);
+                E[2] += w * static_cast<double>(gz[node]);
+            }
+            const float* b = reinterpret_cast<const float*>(pf) + quad_slot(s);
             fxi = b[0]; fyi = b[2]; fzi = b[4];
         }
         const int z0 = max(ck - pp.r2, 0), z1 = min(ck + pp.r2, g.n2 - 2);
@@ -941,7 +963,7 @@ __global__ void __launch_bounds__(kGatherBlock, 8) k_sc_gather_f32(MeshGeom g, P
         const float2 FX = make_float2(fxi, fxi), FY = make_float2(fyi, fyi), FZ = make_float2(fzi, fzi);
         const float2 INV = make_float2(pp.inv_drf, pp.inv_drf), EPS = make_float2(pp.eps2f, pp.eps2f);
         const float2 US = make_float2(pp.pu_s, pp.pu_s);
-        float2 E2x = make_float2(0.f, 0.f), E2y = E2x, E2z = E2x;
+        float Ef[3] = {0.f, 0.f, 0.f};
         const int ncol = (2 * pp.r0 + 1) * (2 * pp.r1 + 1);
         int dcx = -pp.r0, dcy = -pp.r1 + static_cast<int>(jl);    // this lane's next column
         for (int c0 = 0; c0 < ncol; c0 += kGatherLanes) {
@@ -969,15 +991,16 @@ __global__ void __launch_bounds__(kGatherBlock, 8) k_sc_gather_f32(MeshGeom g, P
 #pragma unroll 1
             for (int q = 0; q < kGatherLanes; ++q) {
                 const uint32_t a = __shfl_sync(full, sa, q, kGatherLanes), e = __shfl_sync(full, sb, q, kGatherLanes);
-                for (uint32_t k2 = (a & ~1u) + 2u * jl; k2 < e; k2 += 2u * kGatherLanes) {
-                    // partners k2 and k2 + 1
-                    const float4 xy = pf[k2], zq = pf[k2 + 1u];
+                // partners s0 and s0 + 2 of the lane's parity
+                for (uint32_t s0 = (a & ~3u) + jl; s0 < e; s0 += 4u) {
+                    const float4* q4 = pf + ((s0 & ~3u) + 2u * jl);
+                    const float4 xy = q4[0], zq = q4[1];
                     const float2 dX = __ffma2_rn(make_float2(xy.x, xy.y), m1, FX);
                     const float2 dY = __ffma2_rn(make_float2(xy.z, xy.w), m1, FY);
                     const float2 dZ = __ffma2_rn(make_float2(zq.x, zq.y), m1, FZ);
                     const float2 r2 = __ffma2_rn(dZ, dZ, __ffma2_rn(dY, dY, __fmul2_rn(dX, dX)));
-                    const bool na = k2 >= a && r2.x < pp.rc2f && r2.x >= pp.min_d2f;
-                    const bool nb = k2 + 1u < e && r2.y < pp.rc2f && r2.y >= pp.min_d2f;
+                    const bool na = s0 >= a && r2.x < pp.rc2f && r2.x >= pp.min_d2f;
+                    const bool nb = s0 + 2u >= a && s0 + 2u < e && r2.y < pp.rc2f && r2.y >= pp.min_d2f;
                     const float2 ri = make_float2(rsqrt_hw(r2.x), rsqrt_hw(r2.y));
                     const float2 re = __fadd2_rn(r2, EPS);
                     const float2 rc = make_float2(rcp_hw(re.x), rcp_hw(re.y));
@@ -1003,30 +1026,23 @@ __global__ void __launch_bounds__(kGatherBlock, 8) k_sc_gather_f32(MeshGeom g, P
                     // kc q_j times that (zq.zw = kc q)
                     const float2 f = __fmul2_rn(gsr, make_float2(zq.z, zq.w));
                     const float2 sc = make_float2(na ? f.x : 0.f, nb ? f.y : 0.f);
-                    E2x = __ffma2_rn(dX, sc, E2x);
-                    E2y = __ffma2_rn(dY, sc, E2y);
-                    E2z = __ffma2_rn(dZ, sc, E2z);
+                    Ef[0] = fmaf(dX.y, sc.y, fmaf(dX.x, sc.x, Ef[0]));
+                    Ef[1] = fmaf(dY.y, sc.y, fmaf(dY.x, sc.x, Ef[1]));
+                    Ef[2] = fmaf(dZ.y, sc.y, fmaf(dZ.x, sc.x, Ef[2]));
                 }
             }
         }
-        float Ef[3] = {E2x.x + E2x.y, E2y.x + E2y.y, E2z.x + E2z.y};
 #pragma unroll
-        for (int o = 1; o < kGatherLanes; o <<= 1) {
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                Ef[c] += __shfl_xor_sync(full, Ef[c], o);
-                E[c] += __shfl_xor_sync(full, E[c], o);
-            }
-        }
-#pragma unroll
-        for (int c = 0; c < 3; ++c) E[c] += static_cast<double>(Ef[c]);
+        for (int c = 0; c < 3; ++c) E[c] += static_cast<double>(Ef[c] + __shfl_xor_sync(full, Ef[c], 1));
     }
-    // lane c writes component c
     if (in_range) {
         const uint32_t i = vals[s];
-        if (jl == 0u) ex[i] = act ? E[0] : 0.0;
-        else if (jl == 1u) ey[i] = act ? E[1] : 0.0;
-        else if (jl == 2u) ez[i] = act ? E[2] : 0.0;
+        if (jl == 0u) {
+            ex[i] = act ? E[0] : 0.0;
+            ez[i] = act ? E[2] : 0.0;
+        } else {
+            ey[i] = act ? E[1] : 0.0;
+        }
     }
 }
 
@@ -1275,8 +1291,8 @@ int sc_create(const icb_spacecharge_config& c, uint64_t n_ions, bool pp_float, c
     SC_CUDA(dev_alloc(&S.vals_sorted, S.cap));
     SC_CUDA(dev_alloc(&S.start, static_cast<size_t>(g.ncell) + 1));
     SC_CUDA(dev_alloc(&S.ps, S.cap));
-    SC_CUDA(dev_alloc(&S.pf, static_cast<size_t>(S.cap) + 1));
-    SC_CUDA(cudaMemsetAsync(S.pf, 0, (static_cast<size_t>(S.cap) + 1) * sizeof(float4), s));
+    SC_CUDA(dev_alloc(&S.pf, static_cast<size_t>(S.cap) + 3));       // whole quads
+    SC_CUDA(cudaMemsetAsync(S.pf, 0, (static_cast<size_t>(S.cap) + 3) * sizeof(float4), s));
     if (iso) {
         std::vector<double> tab(kPPTable + 1);
         const double a = S.pp.alpha;
@@ -1428,8 +1444,8 @@ int sc_set_peers(SpaceChargeSolver* S, const double* xyzq, uint64_t n, uint64_t 
         SC_CUDA(dev_alloc(&S->vals, cap));
         SC_CUDA(dev_alloc(&S->vals_sorted, cap));
         SC_CUDA(dev_alloc(&S->ps, cap));
-        SC_CUDA(dev_alloc(&S->pf, static_cast<size_t>(cap) + 1));
-        SC_CUDA(cudaMemsetAsync(S->pf, 0, (static_cast<size_t>(cap) + 1) * sizeof(float4), s));
+        SC_CUDA(dev_alloc(&S->pf, static_cast<size_t>(cap) + 3));
+        SC_CUDA(cudaMemsetAsync(S->pf, 0, (static_cast<size_t>(cap) + 3) * sizeof(float4), s));
         SC_CUDA(dev_alloc(&S->own_flag, cap));
         SC_CUDA(dev_alloc(&S->own_pos, cap));
         SC_CUDA(dev_alloc(&S->own_slots, S->own_cap));

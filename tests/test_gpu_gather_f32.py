@@ -1,4 +1,4 @@
-"""The single-precision gather (four lanes per ion, eight ions per warp) at
+"""The single-precision gather (two lanes per ion, sixteen ions per warp) at
 the sizes where its grouping can go wrong: fewer ions than a warp holds, one
 more and one less than a warp's and a block's ions, ions in the mesh's
 corners (neighbour columns cut by the mesh), excluded ions between others,
@@ -43,7 +43,7 @@ def _lattice(n, lo, hi, seed):
 
 
 @pytest.mark.parametrize("cutoff,alpha", [(2.0, 1.0), (0.7, 2.5), (3.4, 1.0)])
-@pytest.mark.parametrize("n", [2, 7, 8, 9, 31, 32, 33, 257])
+@pytest.mark.parametrize("n", [2, 7, 8, 9, 15, 16, 17, 31, 32, 33, 64, 257])
 def test_gather_matches_oracle_at_group_edges(n, cutoff, alpha):
     mesh = (20, 16, 12)
     lo, hi = np.array([-6e-3, -4.8e-3, -3.6e-3]), np.array([6e-3, 4.8e-3, 3.6e-3])
@@ -59,3 +59,23 @@ def test_gather_matches_oracle_at_group_edges(n, cutoff, alpha):
     rms = np.sqrt(np.mean(np.sum(want ** 2, axis=0)))
     assert np.max(np.abs(got - want)) <= 1e-4 * rms
     assert np.all(got[:, act == 0] == 0.0)
+
+
+def test_an_excluded_ion_without_a_position_changes_nothing():
+    """Four ions share a group of slots: an excluded one that holds no number
+    must add exactly nothing to the others in its group."""
+    mesh = (20, 16, 12)
+    lo, hi = np.array([-6e-3, -4.8e-3, -3.6e-3]), np.array([6e-3, 4.8e-3, 3.6e-3])
+    x, y, z, q = _lattice(30, lo, hi, seed=3)
+    act = np.ones(30, dtype=np.uint8)
+    act[[4, 11, 20]] = 0
+    fields = []
+    for bad in (False, True):
+        if bad:
+            x[4], y[11], z[20] = np.nan, np.inf, -np.inf
+        with Simulation([_field_free()], precision=capi.PREC_MIXED, collision=capi.COLLISION_NONE, rng_seed=1) as sim:
+            sim.upload(_state(x, y, z, q, act))
+            sim.configure_space_charge(capi.SC_P3M_ISOLATED, mesh, lo, hi, alpha_h=1.0, pp_cutoff_cells=2.0)
+            fields.append(sim.space_charge_field())
+    assert np.all(np.isfinite(fields[1]))
+    assert np.array_equal(fields[0], fields[1])
