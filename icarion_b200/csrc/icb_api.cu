@@ -806,11 +806,16 @@ int use_tab(const icb_handle* h, uint32_t K, cudaStream_t st, bool& use) {
     return ICB_OK;
 }
 
-// Room for the per-step field tables of launches of up to K steps (all
-// ensembles, plus the time sequences); allocates outside stream capture only.
+// Doubles of the per-step field tables of launches of up to K steps (all
+// ensembles, plus the time sequences).
+size_t tf_tab_size(const icb_handle* h, uint32_t K) {
+    return h->ens.size() * (static_cast<size_t>(K) + 1u) * (tf_stride(h) + 1u);
+}
+
+// Room for those tables; allocates outside stream capture only.  Without the
+// memory an RF-only handle is left without a table.
 int ensure_tf_tab(icb_handle* h, uint32_t K, cudaStream_t st) {
-    const size_t rows = static_cast<size_t>(K) + 1u;
-    const size_t need = h->ens.size() * rows * (tf_stride(h) + 1u);
+    const size_t need = tf_tab_size(h, K);
     if (h->tf_tab.n >= need) return ICB_OK;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     ICB_CUDA(cudaStreamIsCapturing(st, &cs));
@@ -823,8 +828,14 @@ int ensure_tf_tab(icb_handle* h, uint32_t K, cudaStream_t st) {
     if (h->copy_stream) ICB_CUDA(cudaStreamSynchronize(h->copy_stream));
     if (h->copy_back_stream) ICB_CUDA(cudaStreamSynchronize(h->copy_back_stream));
     for (cudaStream_t cs2 : h->chunk_streams) ICB_CUDA(cudaStreamSynchronize(cs2));
-    ICB_CUDA(h->tf_tab.alloc(need));
-    h->drop_graph();
+    h->drop_graph();               // before its table goes, also when the allocation fails
+    const cudaError_t e = h->tf_tab.alloc(need);
+    if (e == cudaErrorMemoryAllocation && !h->any_tf) {
+        // an RF-only handle steps without a table (its lanes evaluate the cosines)
+        cudaGetLastError();
+        return ICB_OK;
+    }
+    ICB_CUDA(e);
     return ICB_OK;
 }
 
@@ -834,8 +845,11 @@ int ensure_tf_tab(icb_handle* h, uint32_t K, cudaStream_t st) {
 // `use` tells whether the launch has a table.
 int enqueue_tf_tables(icb_handle* h, uint32_t K, cudaStream_t st, bool& use) {
     if (int r = use_tab(h, K, st, use)) return r;
+    if (h->own_capture && !h->any_tf && h->tf_tab.n < tf_tab_size(h, K)) use = false;   // no memory for it before the capture
     if (!use) return ICB_OK;
     if (int r = ensure_tf_tab(h, K, st)) return r;
+    use = h->tf_tab.n >= tf_tab_size(h, K);
+    if (!use) return ICB_OK;
     const uint32_t stride = tf_stride(h);
     const int n_ens = static_cast<int>(h->ens.size());
     double* tseq = h->tf_tab.p + h->ens.size() * (static_cast<size_t>(K) + 1u) * stride;
