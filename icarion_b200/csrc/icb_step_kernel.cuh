@@ -2057,8 +2057,10 @@ __global__ void __launch_bounds__(128, MIN_BLOCKS) k_step(const __grid_constant_
                 if (left == 0u) {
                     uint32_t n = K - kk, ne = 0xFFFFFFFFu;
                     if constexpr (kSkip) {
+                        // (0: an event of the step before, which this lane has
+                        // missed; n stays at least 1, so m - 1 below does)
                         ne = nk + 1u - kk;
-                        if (ne < n) n = ne;
+                        if (ne != 0u && ne < n) n = ne;
                     }
                     const R sd = (m_fabs(v[0] + ah0) + m_fabs(v[1] + ah1) + m_fabs(v[2] + ah2)) * dt_r;
                     auto bound = [&](uint32_t j) {

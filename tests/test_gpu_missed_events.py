@@ -1,0 +1,90 @@
+"""Ions whose stored clock event was not taken when its step went by: they
+were inactive then (icb_update_state, icb_advance_host), the engine clock was
+moved past it (icb_set_clock), or the caller's step left collisions out
+(push and finalize without collide).
+
+The planned FP64 loop (launches of 8 steps or more) and the loop with
+per-step bookkeeping (up to 7) give the same bits from such a state on."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from icarion_b200 import _capi as capi
+from icarion_b200 import config as cfg
+from icarion_b200.sim import Simulation, device_count, generate_ions
+
+pytestmark = pytest.mark.gpu
+
+STATE = ("x", "y", "z", "vx", "vy", "vz", "active", "t_death", "t_arrival")
+COUNTS = ("candidates", "collisions", "rate_overflows", "deaths", "arrivals")
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _gpu():
+    assert device_count() > 0, "these tests need a CUDA device"
+
+
+def _domain(mix=False):
+    # 100 Pa of N2: a candidate event every 14 steps
+    env = {"temperature_K": 300.0, "pressure_Pa": 100.0, "gas_species": "N2"}
+    if mix:
+        env["gas_mixture"] = [{"species": "N2", "mole_fraction": 0.7}, {"species": "He", "mole_fraction": 0.3}]
+    dom = {"instrument": "IMS", "geometry": {"origin_m": [0.0, 0.0, -0.02], "length_m": 0.04, "radius_m": 0.02},
+           "env": env, "fields": {"DC": {"EN_Td": 20.0}}}
+    return cfg.ensemble_params(dom, 150e-20, 4e-9)
+
+
+def _ions(n=300):
+    return generate_ions(21, [cfg.species_spec(n, 200.0 * cfg.AMU_TO_KG, cfg.ELEM_CHARGE_C,
+                                               {"type": "gaussian", "center": [0, 0, 0], "std": [3e-4] * 3},
+                                               {"type": "thermal", "temperature_K": 300.0})])
+
+
+def _miss(sim, how, steps):
+    """Lets the events of `steps` steps go by for every second ion, or for all."""
+    if how == "clock":
+        step, t = sim.clock()
+        sim.set_clock(step + steps, t + steps * 4e-9)
+    elif how == "uncollided":
+        for _ in range(steps):
+            sim.step_batch()
+            sim.finalize()
+    else:
+        idle = sim.download()
+        idle.active[::2] = 0
+        sim.update_state(idle)
+        if how == "host":
+            sim.advance_host(idle, steps, n_chunks=2)
+        else:
+            sim.advance(steps)
+            idle = sim.download()
+        idle.active[:] = 1
+        if how == "update":
+            sim.update_state(idle)
+        else:
+            sim.advance_host(idle, 9, n_chunks=2)
+
+
+def _run(per_launch, how, missed, precision=capi.PREC_FP64, collision=capi.COLLISION_HSS, mix=False):
+    with Simulation([_domain(mix)], precision=precision, collision=collision, rng_seed=5,
+                    steps_per_launch=per_launch) as sim:
+        sim.upload(_ions())
+        sim.advance(30)
+        _miss(sim, how, missed)
+        rs = sim.advance(200)
+        return sim.download(), rs
+
+
+@pytest.mark.parametrize("collision,mix", [(capi.COLLISION_HSS, False), (capi.COLLISION_HSS, True),
+                                           (capi.COLLISION_LANGEVIN, False)])
+@pytest.mark.parametrize("missed", [1, 2, 40])
+@pytest.mark.parametrize("how", ["update", "host", "clock", "uncollided"])
+def test_planned_steps_equal_single_steps_after_missed_events(how, missed, collision, mix):
+    b, rb = _run(7, how, missed, collision=collision, mix=mix)
+    for per_launch in (8, 1000):
+        a, ra = _run(per_launch, how, missed, collision=collision, mix=mix)
+        for k in STATE:
+            np.testing.assert_array_equal(getattr(a, k), getattr(b, k), err_msg=k)
+        for k in COUNTS:
+            assert ra[k] == rb[k], k
