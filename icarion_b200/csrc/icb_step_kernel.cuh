@@ -1750,8 +1750,12 @@ __global__ void __launch_bounds__(128, MIN_BLOCKS) k_step(const __grid_constant_
     }
     if constexpr (kSkip) {
         // restart from the velocity before this step's push (the unfused
-        // push call restarts for the collide call that follows)
-        if (live && (do_coll || do_push) && g_next == kNeedRestart) clock_restart(step0);
+        // push call restarts for the collide call that follows).  An event
+        // before the launch was missed (the ion was inactive at its step, the
+        // engine clock was moved past it, or the caller's step left
+        // collisions out): the optical depth still left runs from here on.
+        const bool missed = static_cast<int32_t>((g_next & ~kRefresh) - step0) < 0;
+        if (live && (do_coll || do_push) && (g_next == kNeedRestart || missed)) clock_restart(step0);
     }
 
     // exact finalize of a step that started at time ts with z = zo
@@ -2057,8 +2061,9 @@ __global__ void __launch_bounds__(128, MIN_BLOCKS) k_step(const __grid_constant_
                 if (left == 0u) {
                     uint32_t n = K - kk, ne = 0xFFFFFFFFu;
                     if constexpr (kSkip) {
-                        // (0: an event of the step before, which this lane has
-                        // missed; n stays at least 1, so m - 1 below does)
+                        // (at least 1: no live lane's event lies before its
+                        // step; n stays at least 1 whatever it holds, so that
+                        // m - 1 below does not wrap)
                         ne = nk + 1u - kk;
                         if (ne != 0u && ne < n) n = ne;
                     }

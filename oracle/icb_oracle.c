@@ -1287,7 +1287,9 @@ int orc_run(const orc_domain* d, int integrator, int collision, uint64_t seed,
                 sk.next = clk_next[i];
                 sk.start = clk_start[i];
                 skip_setup(&sk, d, &Gi, q, m);
-                if (act && contains(d, p) && sk.next == ORC_NEED_RESTART) {
+                /* also when the event lies before the call (missed) */
+                const int missed = (int32_t)((sk.next & ~ORC_REFRESH) - (uint32_t)step0) < 0;
+                if (act && contains(d, p) && (sk.next == ORC_NEED_RESTART || missed)) {
                     uint64_t ov = 0;
                     skip_restart(&sk, &Gi, v, (uint32_t)step0, &ov);
                     ovf_tot += ov;

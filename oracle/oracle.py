@@ -163,7 +163,7 @@ def build() -> None:
 def lib() -> C.CDLL:
     global _lib
     if _lib is None:
-        if not LIB.exists():
+        if not LIB.exists() or LIB.stat().st_mtime < (HERE / "icb_oracle.c").stat().st_mtime:
             build()
         L = C.CDLL(str(LIB))
         DP = C.POINTER(C.c_double)
