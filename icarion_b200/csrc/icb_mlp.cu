@@ -56,6 +56,29 @@ __device__ __forceinline__ void cp_async16(float* dst, const float* src) {
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
+// Loads of what the previous kernel of a programmatic launch chain wrote.
+// That kernel may still run when this one starts, so the data is not
+// read-only for this kernel's life: no const __restrict__ pointer (which
+// allows the non-coherent path, and a load above the wait), but volatile
+// ordinary loads, which stay behind cudaGridDependencySynchronize and see
+// all that the kernels before it wrote.
+__device__ __forceinline__ float ld_after(const float* p) {
+    float v;
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float2 ld_after2(const float* p) {
+    float2 v;
+    asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float4 ld_after4(const float* p) {
+    float4 v;
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+
 // Forward of one sample in FP32 arithmetic (optionally with BF16-rounded
 // weights and first-layer activations); h1, h2 receive the activations.
 template <bool BF16>
@@ -88,7 +111,7 @@ __device__ float mlp_forward_one(const float* w, float x0, float x1, float* h1, 
 // dependent chains of 64 FMAs; 16 samples a block spread it over 64 SMs (one
 // thread per sample in 8 blocks took 104 us).
 template <bool BF16>
-__global__ void __launch_bounds__(kSThreads) k_mlp_samples(const float* __restrict__ params,
+__global__ void __launch_bounds__(kSThreads) k_mlp_samples(const float* params,
                                                            const float* __restrict__ x, const float* __restrict__ y,
                                                            const uint32_t* __restrict__ perm, uint64_t first,
                                                            uint32_t count, float inv_batch, uint32_t ld,
@@ -121,12 +144,18 @@ __global__ void __launch_bounds__(kSThreads) k_mlp_samples(const float* __restri
     float4 wv[kMlpH * kMlpH / 4 / kSThreads];
 #pragma unroll
     for (int j = 0; j < kMlpH * kMlpH / 4 / kSThreads; ++j)
-        wv[j] = *reinterpret_cast<const float4*>(params + kMlpOffW2 + 4 * (tid + j * kSThreads));
-    float b2v[4];
+        wv[j] = ld_after4(params + kMlpOffW2 + 4 * (tid + j * kSThreads));
+    float b1v[4], b2v[4];
+    float2 w1v[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) b2v[j] = params[kMlpOffB2 + q + 16 * j];
-    const float b3v = params[kMlpOffB3];
-    if (tid < kMlpH) w3[tid] = params[kMlpOffW3 + tid];
+    for (int j = 0; j < 4; ++j) {
+        const int c = q + 16 * j;
+        b1v[j] = ld_after(params + kMlpOffB1 + c);
+        b2v[j] = ld_after(params + kMlpOffB2 + c);
+        w1v[j] = ld_after2(params + kMlpOffW1 + 2 * c);
+    }
+    const float b3v = ld_after(params + kMlpOffB3);
+    if (tid < kMlpH) w3[tid] = ld_after(params + kMlpOffW3 + tid);
 #pragma unroll
     for (int j = 0; j < kMlpH * kMlpH / 4 / kSThreads; ++j) {
         const int e = 4 * (tid + j * kSThreads);
@@ -140,9 +169,9 @@ __global__ void __launch_bounds__(kSThreads) k_mlp_samples(const float* __restri
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         const int c = q + 16 * j;
-        float w0 = params[kMlpOffW1 + 2 * c], w1 = params[kMlpOffW1 + 2 * c + 1];
+        float w0 = w1v[j].x, w1 = w1v[j].y;
         if (BF16) { w0 = bf16r(w0); w1 = bf16r(w1); }
-        float a = tanhf(fmaf(w0, x0, fmaf(w1, x1, params[kMlpOffB1 + c])));
+        float a = tanhf(fmaf(w0, x0, fmaf(w1, x1, b1v[j])));
         if (BF16) a = bf16r(a);
         H1[s * kWs + c] = valid ? a : 0.f;
     }
@@ -253,8 +282,8 @@ struct AdamState {
 // SM reads more than 72 KB of the samples' 1 MB (9.2 us with cold caches;
 // reading the samples in place, strided, took 16 us, and unit-major rows 14.5).
 template <bool ADAM>
-__global__ void __launch_bounds__(kUThreads) k_mlp_update(const float* __restrict__ rows,
-                                                          const float* __restrict__ cols, uint32_t ld, int ngroups,
+__global__ void __launch_bounds__(kUThreads) k_mlp_update(const float* rows, const float* cols,
+                                                          uint32_t ld, int ngroups,
                                                           int first_chunk, int last_chunk,
                                                           float* __restrict__ gsum_buf,
                                                           double* __restrict__ lsum_buf,
@@ -371,14 +400,13 @@ __global__ void __launch_bounds__(kUThreads) k_mlp_update(const float* __restric
         } else if (tid < 2 * kUGroups) {
             const int b = tid >> 1;
             if (b < ng) {
-                const float4* e4 = reinterpret_cast<const float4*>(
-                    cols + static_cast<size_t>((tid & 1) ? kColErr : kColDout) * ld +
-                    static_cast<size_t>(g0 + b) * kGroup);
+                const float* e1 = cols + static_cast<size_t>((tid & 1) ? kColErr : kColDout) * ld +
+                                  static_cast<size_t>(g0 + b) * kGroup;
                 float acc = 0.f;
                 double lacc = 0.0;
 #pragma unroll 32
                 for (int s = 0; s < kGroup / 4; ++s) {
-                    const float4 e = e4[s];
+                    const float4 e = ld_after4(e1 + 4 * s);
                     if (tid & 1) {
                         lacc += static_cast<double>(e.x) * e.x;
                         lacc += static_cast<double>(e.y) * e.y;
