@@ -17,6 +17,9 @@ cudaError_t launch_tf_table(const StepParams& p, double* tab, double* tseq, uint
 // The FP64 forms' table of functions of a 16-bit draw on the current device
 // (1.5 MB of module memory), filled on `s` where it is not yet.
 cudaError_t launch_angle_table(const double2** tab, cudaStream_t s);
+// Unique id of the calling thread's current context (another one after a
+// device reset), or 0 when it cannot be had.
+unsigned long long current_context_id();
 // The device engine clock K steps on (step_dev, t_dev).
 cudaError_t launch_clock_advance(unsigned long long* step, double* t, const double* dt, int n_ens, uint32_t K,
                                  cudaStream_t s);

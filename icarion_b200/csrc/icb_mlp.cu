@@ -505,20 +505,24 @@ struct DevVec {
 // workspace cost 0.6 ms on the host, more than half of a short training run;
 // the pool hands the same memory to the next call in a few microseconds.  It
 // keeps at most kCallPoolKeep bytes per device between calls (the driver
-// releases the rest when a call's stream is synchronised), belongs to no
-// handle, and is safe with several threads and streams: allocations are
-// stream ordered and the driver orders their reuse.  Null when the device
-// has no pools or the creation fails (the caller then allocates plainly).
+// releases the rest when a stream is synchronised after a free: each call
+// does so last), belongs to no handle, and is safe with several threads and
+// streams: allocations are stream ordered and the driver orders their reuse.
+// Null when the device has no pools or the creation fails (the caller then
+// allocates plainly).  A device reset takes the pool with its context: it is
+// used only in the context it was made in, known by the context's id.
 constexpr uint64_t kCallPoolKeep = 32ull << 20;
 static cudaMemPool_t call_pool(int device) {
     static std::mutex m;
     static cudaMemPool_t pools[64] = {};
+    static unsigned long long ctxs[64] = {};
     if (device < 0 || device >= 64) return nullptr;
+    const unsigned long long ctx = current_context_id();
+    if (ctx == 0) return nullptr;
     std::lock_guard<std::mutex> lock(m);
+    if (pools[device] && ctxs[device] == ctx) return pools[device];
+    pools[device] = nullptr;
     uint64_t keep = kCallPoolKeep;
-    // (setting the threshold also finds out whether a device reset took the pool)
-    if (pools[device] && cudaMemPoolSetAttribute(pools[device], cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess)
-        return pools[device];
     cudaMemPoolProps props{};
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;
@@ -531,6 +535,7 @@ static cudaMemPool_t call_pool(int device) {
         return nullptr;
     }
     pools[device] = pool;
+    ctxs[device] = ctx;
     return pool;
 }
 
@@ -626,8 +631,14 @@ struct CallMem {
     bool pooled = false;
     ~CallMem() {
         if (!p) return;
-        if (pooled) cudaFreeAsync(p, s);
-        else cudaFree(p);
+        if (!pooled) {
+            cudaFree(p);
+            return;
+        }
+        // the pool gives back what it holds above its bound at a
+        // synchronisation after the free; the call's work is done by now
+        cudaFreeAsync(p, s);
+        cudaStreamSynchronize(s);
     }
     cudaError_t alloc(size_t bytes, int device, cudaStream_t stream) {
         s = stream;

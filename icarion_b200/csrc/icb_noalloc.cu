@@ -50,9 +50,9 @@ std::mutex g_scratch_mutex;
 using CtxGetCurrentFn = int (*)(void** ctx);
 using CtxGetIdFn = int (*)(void* ctx, unsigned long long* id);
 
-// Unique id of the calling thread's current context, or 0 when it cannot be
-// had (the caller then looks the address up on every call).
-unsigned long long current_context_id() {
+}  // namespace
+
+unsigned long long icb::current_context_id() {
     static CtxGetCurrentFn get_current = nullptr;
     static CtxGetIdFn get_id = nullptr;
     static std::once_flag once;
@@ -73,6 +73,8 @@ unsigned long long current_context_id() {
     if (get_current(&ctx) != 0 || !ctx || get_id(ctx, &id) != 0) return 0;
     return id;
 }
+
+namespace {
 
 // Makes `device` current for the lifetime of the guard and gives the
 // caller's current device back on every return path.
@@ -178,7 +180,7 @@ extern "C" int icb_moments_noalloc(int device, uint64_t n, const double* x, cons
     double* scratch = nullptr;
     {
         std::lock_guard<std::mutex> lock(g_scratch_mutex);
-        const unsigned long long ctx = current_context_id();
+        const unsigned long long ctx = icb::current_context_id();   // 0: looked up on every call
         if (!g_scratch_addr[device] || ctx == 0 || ctx != g_scratch_ctx[device]) {
             // First call in this device's context: resolve the scratch
             // array's device address with the device current.

@@ -449,7 +449,9 @@ typedef struct icb_mlp_train_config {
 /* Xavier-uniform initial parameters from `seed`. */
 int icb_mlp_init(uint64_t seed, float* params);
 /* Adam on the mean squared error over n samples (x: 2n floats, y: n floats,
- * host); params in/out; loss_per_epoch (epochs doubles) may be NULL. */
+ * host); params in/out; loss_per_epoch (epochs doubles) may be NULL.
+ * Training and gradient calls take their device workspace from a pool of the
+ * library, which keeps up to 32 MiB per device until the process ends. */
 int icb_mlp_train(int device, const icb_mlp_train_config* cfg, uint64_t n, const float* x, const float* y,
                   float* params, double* loss_per_epoch);
 /* Network output for n inputs: mode 0 = FP32 reference arithmetic, mode 1 =
