@@ -677,6 +677,8 @@ int build_ens_const(const icb_ensemble_params& P, EnsConst& C, int& field_kind, 
     return ICB_OK;
 }
 
+int size_rf_tab(icb_handle* h);
+
 // Rebuild the time-dependent field table, the ensembles' tf flags and
 // field bounds, and the handle's field kind from the waveforms and TIMS
 // fields set so far; uploads the table when any ensemble uses it.
@@ -771,7 +773,7 @@ int rebuild_time_fields(icb_handle* h) {
         ICB_CUDA(cudaMemcpy(h->tfield.p, tfs.data(), ne * sizeof(TimeField), cudaMemcpyHostToDevice));
     }
     ++h->gen;
-    return ICB_OK;
+    return h->n > 0 ? size_rf_tab(h) : ICB_OK;
 }
 
 inline unsigned grid_for(uint64_t n, int block) { return static_cast<unsigned>((n + block - 1) / block); }
@@ -791,20 +793,6 @@ bool rf_tab(const icb_handle* h, uint32_t K) {
         if (!C.tf && (C.rf || C.ac)) return true;
     return false;
 }
-bool needs_tab(const icb_handle* h, uint32_t K) { return h->any_tf || rf_tab(h, K); }
-
-// needs_tab, but false for an RF-only handle on a stream that its caller is
-// capturing: the lanes then evaluate the cosines, so that a captured graph
-// holds no pointer to a table that a longer later launch replaces (the
-// handle's own graphs are dropped then).
-int use_tab(const icb_handle* h, uint32_t K, cudaStream_t st, bool& use) {
-    use = needs_tab(h, K);
-    if (!use || h->any_tf || h->own_capture) return ICB_OK;
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    ICB_CUDA(cudaStreamIsCapturing(st, &cs));
-    use = cs == cudaStreamCaptureStatusNone;
-    return ICB_OK;
-}
 
 // Doubles of the per-step field tables of launches of up to K steps (all
 // ensembles, plus the time sequences).
@@ -812,8 +800,50 @@ size_t tf_tab_size(const icb_handle* h, uint32_t K) {
     return h->ens.size() * (static_cast<size_t>(K) + 1u) * (tf_stride(h) + 1u);
 }
 
-// Room for those tables; allocates outside stream capture only.  Without the
-// memory an RF-only handle is left without a table.
+// Whether a launch of K steps on `st` reads a table.  An RF-only handle has
+// one if size_rf_tab found the memory for it.  It uses none on a stream that
+// its caller is capturing: the lanes then evaluate the cosines, so that a
+// captured graph holds no pointer to a table that a later upload or field
+// change replaces (the handle's own graphs are dropped then).
+int use_tab(const icb_handle* h, uint32_t K, cudaStream_t st, bool& use) {
+    use = h->any_tf || (rf_tab(h, K) && h->tf_tab.n >= tf_tab_size(h, K));
+    if (!use || h->any_tf || h->own_capture) return ICB_OK;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    ICB_CUDA(cudaStreamIsCapturing(st, &cs));
+    use = cs == cudaStreamCaptureStatusNone;
+    return ICB_OK;
+}
+
+// Waits for every stream of the handle.
+int sync_streams(icb_handle* h) {
+    ICB_CUDA(cudaStreamSynchronize(h->stream));
+    if (h->copy_stream) ICB_CUDA(cudaStreamSynchronize(h->copy_stream));
+    if (h->copy_back_stream) ICB_CUDA(cudaStreamSynchronize(h->copy_back_stream));
+    for (cudaStream_t cs : h->chunk_streams) ICB_CUDA(cudaStreamSynchronize(cs));
+    return ICB_OK;
+}
+
+// The drive table of a handle whose fields depend on time through
+// constant-voltage RF and AC drives only, sized once (at the upload, or when
+// the last waveform is cleared) for its longest launch, so that an advance
+// neither allocates nor waits: 8 (K + 1) x 13 bytes per ensemble, x 25 with
+// RK4 (104 and 200 KB for 1,000 steps).  Without the memory the handle has
+// no table and its lanes evaluate the cosines.
+int size_rf_tab(icb_handle* h) {
+    if (h->any_tf || !rf_tab(h, h->K) || h->tf_tab.n >= tf_tab_size(h, h->K)) return ICB_OK;
+    if (int r = sync_streams(h)) return r;
+    h->drop_graph();
+    const cudaError_t e = h->tf_tab.alloc(tf_tab_size(h, h->K));
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        return ICB_OK;
+    }
+    ICB_CUDA(e);
+    return ICB_OK;
+}
+
+// Room for the tables of a time-dependent field; allocates outside stream
+// capture only.
 int ensure_tf_tab(icb_handle* h, uint32_t K, cudaStream_t st) {
     const size_t need = tf_tab_size(h, K);
     if (h->tf_tab.n >= need) return ICB_OK;
@@ -824,18 +854,9 @@ int ensure_tf_tab(icb_handle* h, uint32_t K, cudaStream_t st) {
     // the old table may still be read by this handle's queued work: wait
     // for the handle's own streams only (not the whole device)
     ICB_CUDA(cudaStreamSynchronize(st));
-    ICB_CUDA(cudaStreamSynchronize(h->stream));
-    if (h->copy_stream) ICB_CUDA(cudaStreamSynchronize(h->copy_stream));
-    if (h->copy_back_stream) ICB_CUDA(cudaStreamSynchronize(h->copy_back_stream));
-    for (cudaStream_t cs2 : h->chunk_streams) ICB_CUDA(cudaStreamSynchronize(cs2));
+    if (int r = sync_streams(h)) return r;
     h->drop_graph();               // before its table goes, also when the allocation fails
-    const cudaError_t e = h->tf_tab.alloc(need);
-    if (e == cudaErrorMemoryAllocation && !h->any_tf) {
-        // an RF-only handle steps without a table (its lanes evaluate the cosines)
-        cudaGetLastError();
-        return ICB_OK;
-    }
-    ICB_CUDA(e);
+    ICB_CUDA(h->tf_tab.alloc(need));
     return ICB_OK;
 }
 
@@ -845,11 +866,10 @@ int ensure_tf_tab(icb_handle* h, uint32_t K, cudaStream_t st) {
 // `use` tells whether the launch has a table.
 int enqueue_tf_tables(icb_handle* h, uint32_t K, cudaStream_t st, bool& use) {
     if (int r = use_tab(h, K, st, use)) return r;
-    if (h->own_capture && !h->any_tf && h->tf_tab.n < tf_tab_size(h, K)) use = false;   // no memory for it before the capture
     if (!use) return ICB_OK;
-    if (int r = ensure_tf_tab(h, K, st)) return r;
-    use = h->tf_tab.n >= tf_tab_size(h, K);
-    if (!use) return ICB_OK;
+    if (h->any_tf) {
+        if (int r = ensure_tf_tab(h, K, st)) return r;
+    }
     const uint32_t stride = tf_stride(h);
     const int n_ens = static_cast<int>(h->ens.size());
     double* tseq = h->tf_tab.p + h->ens.size() * (static_cast<size_t>(K) + 1u) * stride;
@@ -1374,6 +1394,7 @@ int icb_upload_ions(icb_handle* h, uint64_t n,
         ICB_CUDA(h->stage.alloc(f64 ? 0 : 3 * n));   // a third per axis
         h->n = n;
     }
+    if (int r = size_rf_tab(h)) return r;   // after the ions: it can do without
     h->first_id = first_ion_id;
     ++h->gen;
     h->ens_off = off;
@@ -1555,7 +1576,7 @@ int icb_advance(icb_handle* h, uint64_t n_steps, icb_run_stats* stats) {
             // not allowed on the legacy default stream); replayed on h->stream.
             cudaGraph_t g = nullptr;
             const uint32_t Kg = h->sc ? 1u : static_cast<uint32_t>(std::min<uint64_t>(n_steps, h->K));
-            if (needs_tab(h, Kg)) {
+            if (h->any_tf) {
                 if (int r = ensure_tf_tab(h, Kg, s)) return r;
             }
             ICB_CUDA(cudaStreamBeginCapture(h->own_stream, cudaStreamCaptureModeThreadLocal));
