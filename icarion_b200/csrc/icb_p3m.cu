@@ -166,9 +166,12 @@ __global__ void __launch_bounds__(kStartThreads) k_sc_cell_start(const uint32_t*
 // four slots 4k .. 4k + 3 the even two's and then the odd two's as two float4
 // each, {x0, x2, y0, y2}, {z0, z2, kq0, kq2}: a lane that owns one parity
 // loads what the packed (two-wide) FP32 instructions take.
-__device__ __forceinline__ uint32_t quad_slot(uint32_t s) {
-    return 16u * (s >> 2) + 8u * (s & 1u) + ((s >> 1) & 1u);
+// quad_slot: the float that holds slot s's x (past 32 bits from 2^30 slots on).
+__host__ __device__ constexpr size_t quad_slot(uint32_t s) {
+    return 16 * static_cast<size_t>(s >> 2) + 8u * (s & 1u) + ((s >> 1) & 1u);
 }
+static_assert(quad_slot(6u) == 17 && quad_slot(1u << 30) == size_t(1) << 32 && quad_slot(0x7fffffffu) < size_t(1) << 33,
+              "four floats a slot, up to 2^31 - 1 slots");
 __global__ void k_sc_permute(MeshGeom g, const double* __restrict__ x, const double* __restrict__ y,
                              const double* __restrict__ z, const double* __restrict__ q,
                              const uint32_t* __restrict__ vals, uint32_t n, uint32_t n_own, PeerIons peers,
