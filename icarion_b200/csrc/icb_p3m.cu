@@ -1459,6 +1459,9 @@ int sc_set_peers(SpaceChargeSolver* S, const double* xyzq, uint64_t n, uint64_t 
         S->scan_bytes = 0;
         SC_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, S->scan_bytes, S->own_flag, S->own_pos, static_cast<int>(cap), s));
         SC_CUDA(cudaMalloc(&S->scan_tmp, std::max<size_t>(S->scan_bytes, 16)));
+        // pf is cleared before this returns: the next solve may run on
+        // another stream (icb_set_stream does not wait)
+        SC_CUDA(cudaStreamSynchronize(s));
     }
     S->peers.xyzq = reinterpret_cast<const double4*>(xyzq);
     S->peers.n = static_cast<uint32_t>(n);
