@@ -39,6 +39,7 @@ int fail(int code, const char* fmt, ...) {
     do {                                                                                 \
         cudaError_t err_ = (call);                                                       \
         if (err_ != cudaSuccess) {                                                       \
+            cudaGetLastError();   /* not to be found by a later launch's check */        \
             return fail(err_ == cudaErrorMemoryAllocation ? ICB_ERR_OUT_OF_MEMORY        \
                                                           : ICB_ERR_CUDA,                \
                         "%s failed: %s (%s:%d)", #call, cudaGetErrorString(err_),        \
@@ -1374,6 +1375,7 @@ int icb_upload_ions(icb_handle* h, uint64_t n,
     }
     ICB_CUDA(cudaStreamSynchronize(h->stream));
     if (h->n != n) {
+        h->n = 0;                  // no ions until every array is there
         const bool f64 = h->fp64(), hl = h->hilo();
         ICB_CUDA(h->x.alloc(hl ? 0 : n)); ICB_CUDA(h->y.alloc(hl ? 0 : n)); ICB_CUDA(h->z.alloc(hl ? 0 : n));
         ICB_CUDA(h->xh.alloc(hl ? n : 0)); ICB_CUDA(h->xl.alloc(hl ? n : 0));

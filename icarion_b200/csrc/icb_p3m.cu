@@ -1203,6 +1203,7 @@ struct SpaceChargeSolver {
         cudaError_t e_ = (expr);                                                               \
         if (e_ != cudaSuccess) {                                                               \
             err = std::string(#expr) + ": " + cudaGetErrorString(e_);                          \
+            cudaGetLastError();   /* not to be found by a later launch's check */              \
             return e_ == cudaErrorMemoryAllocation ? ICB_ERR_OUT_OF_MEMORY : ICB_ERR_CUDA;     \
         }                                                                                      \
     } while (0)
@@ -1414,13 +1415,14 @@ int sc_set_peers(SpaceChargeSolver* S, const double* xyzq, uint64_t n, uint64_t 
                  cudaStream_t s, std::string& err) {
     if (n == 0) {
         S->peers = PeerIons{};
-        return ICB_OK;
+        if (S->cap != 0) return ICB_OK;
+        skip_b = skip_n = 0;               // the own ions' buffers, given up below for a growth that failed
     }
     if (S->mode != ICB_SC_P3M_ISOLATED) {
         err = "peer ions need the isolated P3M solver";
         return ICB_ERR_UNSUPPORTED;
     }
-    if (xyzq == nullptr || (reinterpret_cast<uintptr_t>(xyzq) & 15u) != 0u) {
+    if ((n > 0 && xyzq == nullptr) || (reinterpret_cast<uintptr_t>(xyzq) & 15u) != 0u) {
         err = "peer ions: null or misaligned device array (16-byte aligned x, y, z, q quadruples)";
         return ICB_ERR_INVALID_ARGUMENT;
     }
@@ -1430,9 +1432,11 @@ int sc_set_peers(SpaceChargeSolver* S, const double* xyzq, uint64_t n, uint64_t 
     }
     const uint64_t total = static_cast<uint64_t>(S->own_cap) + n;
     if (total > S->cap || S->own_slots == nullptr) {
-        // grow the sort, permutation and slot buffers to own + peers
+        // grow the sort, permutation and slot buffers to own + peers; until
+        // all of them are there, a solve has none (cap = 0)
         SC_CUDA(cudaStreamSynchronize(s));
         const uint32_t cap = static_cast<uint32_t>(std::max<uint64_t>(total, S->cap));
+        S->cap = 0;
         for (void** p : {reinterpret_cast<void**>(&S->keys), reinterpret_cast<void**>(&S->keys_sorted),
                          reinterpret_cast<void**>(&S->vals), reinterpret_cast<void**>(&S->vals_sorted),
                          reinterpret_cast<void**>(&S->ps), reinterpret_cast<void**>(&S->pf), &S->cub_tmp,
@@ -1441,7 +1445,6 @@ int sc_set_peers(SpaceChargeSolver* S, const double* xyzq, uint64_t n, uint64_t 
             if (*p) cudaFree(*p);
             *p = nullptr;
         }
-        S->cap = cap;
         SC_CUDA(dev_alloc(&S->keys, cap));
         SC_CUDA(dev_alloc(&S->keys_sorted, cap));
         SC_CUDA(dev_alloc(&S->vals, cap));
@@ -1462,6 +1465,7 @@ int sc_set_peers(SpaceChargeSolver* S, const double* xyzq, uint64_t n, uint64_t 
         // pf is cleared before this returns: the next solve may run on
         // another stream (icb_set_stream does not wait)
         SC_CUDA(cudaStreamSynchronize(s));
+        S->cap = cap;
     }
     S->peers.xyzq = reinterpret_cast<const double4*>(xyzq);
     S->peers.n = static_cast<uint32_t>(n);
@@ -1485,6 +1489,10 @@ int sc_solve(SpaceChargeSolver* S, const double* x, const double* y, const doubl
              const uint8_t* flags, uint64_t n, cudaStream_t s, std::string& err) {
     if (n > S->own_cap) {
         err = "more ions than the space-charge solver was configured for";
+        return ICB_ERR_STATE;
+    }
+    if (S->cap == 0) {
+        err = "the buffers for the peers' ions could not be had: set fewer peers or configure space charge again";
         return ICB_ERR_STATE;
     }
     const MeshGeom& g = S->g;
