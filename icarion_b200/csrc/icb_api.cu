@@ -116,6 +116,10 @@ __global__ void k_to_hilo(const double* __restrict__ src, float* __restrict__ hi
         lo[i] = static_cast<float>(src[i] - static_cast<double>(h));
     }
 }
+__global__ void k_from_float(const float* __restrict__ src, double* __restrict__ dst, uint64_t n) {
+    const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (i < n) dst[i] = static_cast<double>(src[i]);
+}
 __global__ void k_from_hilo(const float* __restrict__ hi, const float* __restrict__ lo, double* __restrict__ dst, uint64_t n) {
     const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i < n) dst[i] = static_cast<double>(hi[i]) + static_cast<double>(lo[i]);
@@ -1393,7 +1397,13 @@ int icb_upload_ions(icb_handle* h, uint64_t n,
         ICB_CUDA(h->t_death.alloc(n)); ICB_CUDA(h->t_arr.alloc(n)); ICB_CUDA(h->birth.alloc(n));
         ICB_CUDA(h->zprev.alloc(n));
         ICB_CUDA(h->flags.alloc(n)); ICB_CUDA(h->active_stage.alloc(n));
-        ICB_CUDA(h->stage.alloc(f64 ? 0 : 3 * n));   // a third per axis
+        // a third per axis, which the overlapped host path needs and a
+        // download converts in one launch; one for all where memory is short
+        // (8 bytes an ion instead of 24)
+        if (h->stage.alloc(f64 ? 0 : 3 * n) == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            ICB_CUDA(h->stage.alloc(n));
+        }
         h->n = n;
     }
     if (int r = size_rf_tab(h)) return r;   // after the ions: it can do without
@@ -1529,9 +1539,9 @@ int icb_download_ions(icb_handle* h, double* x, double* y, double* z,
     for (int a = 0; a < 3; ++a) {
         if (!pos[a]) continue;
         if (h->hilo()) {
-            // (its own third of the staging; the velocities' conversion follows
-            // these copies on the stream)
-            double* st = h->stage.p + static_cast<size_t>(a) * n;
+            // (its own third of the staging if there are three; conversions
+            // follow earlier copies on the stream)
+            double* st = h->stage.p + (h->stage.n >= 3 * n ? static_cast<size_t>(a) * n : 0);
             k_from_hilo<<<g, 256, 0, s>>>(ph[a]->p, pl[a]->p, st, n);
             ICB_CUDA(cudaGetLastError());
             ICB_CUDA(cudaMemcpyAsync(pos[a], st, bytes, cudaMemcpyDeviceToHost, s));
@@ -1543,15 +1553,24 @@ int icb_download_ions(icb_handle* h, double* x, double* y, double* z,
     DevBuf<double>* vd[3] = {&h->vxd, &h->vyd, &h->vzd};
     DevBuf<float>* vf[3] = {&h->vxf, &h->vyf, &h->vzf};
     // velocities and activity bytes: one conversion launch, then the copies
+    // (axis by axis where the staging holds one)
     const bool conv = !h->fp64() && (vel[0] || vel[1] || vel[2]);
-    if (conv || active) {
-        k_chunk_out<<<g, 256, 0, s>>>(conv ? vf[0]->p : nullptr, vf[1]->p, vf[2]->p, h->stage.p, n, h->flags.p,
-                                      h->active_stage.p, n);
+    const bool thirds = h->stage.n >= 3 * n;
+    if ((conv && thirds) || active) {
+        k_chunk_out<<<g, 256, 0, s>>>(conv && thirds ? vf[0]->p : nullptr, vf[1]->p, vf[2]->p, h->stage.p, n,
+                                      h->flags.p, h->active_stage.p, n);
         ICB_CUDA(cudaGetLastError());
     }
     for (int a = 0; a < 3; ++a) {
         if (!vel[a]) continue;
-        const double* src = h->fp64() ? vd[a]->p : h->stage.p + static_cast<size_t>(a) * n;
+        const double* src = vd[a]->p;
+        if (conv && thirds) {
+            src = h->stage.p + static_cast<size_t>(a) * n;
+        } else if (conv) {
+            k_from_float<<<g, 256, 0, s>>>(vf[a]->p, h->stage.p, n);
+            ICB_CUDA(cudaGetLastError());
+            src = h->stage.p;
+        }
         ICB_CUDA(cudaMemcpyAsync(vel[a], src, bytes, cudaMemcpyDeviceToHost, s));
     }
     if (active) ICB_CUDA(cudaMemcpyAsync(active, h->active_stage.p, n, cudaMemcpyDeviceToHost, s));
@@ -2007,6 +2026,15 @@ int icb_advance_host(icb_handle* h, uint64_t n_steps, int n_chunks, double* x, d
         cudaEvent_t e;
         ICB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         h->hev.push_back(e);
+    }
+    if (!f64 && h->stage.n < 3 * n) {
+        // the upload found memory for one array; the old one stays if there
+        // still is none
+        DevBuf<double> three;
+        ICB_CUDA(three.alloc(3 * n));
+        if (int r = sync_streams(h)) return r;
+        std::swap(h->stage.p, three.p);
+        std::swap(h->stage.n, three.n);
     }
     cudaStream_t s = h->stream, cs = h->copy_stream, bs = h->copy_back_stream;
     double* pos[3] = {x, y, z};
