@@ -684,6 +684,35 @@ int build_ens_const(const icb_ensemble_params& P, EnsConst& C, int& field_kind, 
 
 int size_rf_tab(icb_handle* h);
 
+// Launch shape (block, deferred-collision batch per warp, steps per vote)
+// where neither the caller nor icb_autotune chose one.
+void default_shape(icb_handle* h, bool time_fields) {
+    if (h->shape_tuned) return;
+    uint32_t block = 128u, pend = 10u, spv = 8u;      // measured optimum of the mixed event loop
+    if (time_fields) {
+        // the autotuner's optimum on the TIMS workload (64-thread blocks, a
+        // 6-lane deferred batch, 8 steps per vote: 1.05e11 ion-steps/s; 4
+        // steps per vote gave 9.8e10)
+        block = 64u;
+        pend = 6u;
+    } else if (h->fp64() && h->cfg.integrator == ICB_INTEGRATOR_BORIS && h->base_field_kind == kFieldUniform &&
+               !h->magnetic && h->coll != kCollHSSPlain) {
+        // The planned FP64 loop (uniform field, no B): its steps are cheap
+        // next to its events, so the warp votes every 16 steps, and waits for
+        // 16 pending lanes where events are frequent (A <|th|> per step).
+        // 262,144 ions x 1,000 steps, pending / vote: at 1000 Pa (0.085) 10/8
+        // 3050 us, 16/16 2677, 24/16 2678; at 100 Pa (0.0085) 1007, 881
+        // (10/16 879); at 30 Pa 689, 717, 947 (10/16 619).
+        double rate = 0.0;
+        for (const EnsConst& c : h->ens_const) rate = std::max(rate, c.A * c.mean_th);
+        spv = 16u;
+        if (rate >= 0.01) pend = 16u;
+    }
+    if (h->cfg.block_size <= 0) h->block = static_cast<int>(block);
+    if (h->cfg.pending_threshold <= 0) h->pend = pend;
+    if (h->cfg.steps_per_vote <= 0) h->spv = spv;
+}
+
 // Rebuild the time-dependent field table, the ensembles' tf flags and
 // field bounds, and the handle's field kind from the waveforms and TIMS
 // fields set so far; uploads the table when any ensemble uses it.
@@ -761,15 +790,7 @@ int rebuild_time_fields(icb_handle* h) {
             C.Emax = base;
         }
     }
-    if (any != h->any_tf && !h->shape_tuned) {
-        // launch shape of the time-dependent instance where neither the
-        // caller nor icb_autotune chose one: the autotuner's optimum on the
-        // TIMS workload (64-thread blocks, a 6-lane deferred batch, 8 steps
-        // per vote: 1.05e11 ion-steps/s; 4 steps per vote gave 9.8e10)
-        if (h->cfg.block_size <= 0) h->block = any ? 64 : 128;
-        if (h->cfg.pending_threshold <= 0) h->pend = any ? 6u : 10u;
-        if (h->cfg.steps_per_vote <= 0) h->spv = 8u;
-    }
+    if (any != h->any_tf) default_shape(h, any);
     h->any_tf = any;
     h->field_kind = any ? std::max(h->base_field_kind, static_cast<int>(kFieldLinearRF)) : h->base_field_kind;
     if (any) {
@@ -1253,21 +1274,8 @@ int icb_create(const icb_config* cfg, icb_handle** out) {
             return fail(ICB_ERR_INVALID_ARGUMENT, "steps_per_launch must be <= %u", kMaxStepsPerLaunch);
         h->K = static_cast<uint32_t>(cfg->steps_per_launch);
     }
-    // Deferred-collision batch per warp (lanes of 32): measured optimum with
-    // 8 steps per vote.
-    h->pend = 10u;
-    // The planned FP64 loop (uniform field, no B): its steps are cheap next to
-    // its events, so the warp votes every 16 steps, and waits for 16 pending
-    // lanes where events are frequent (A <|th|> per step).  262,144 ions x
-    // 1,000 steps, pending / vote: at 1000 Pa (0.085) 10/8 3050 us, 16/16
-    // 2677, 24/16 2678; at 100 Pa (0.0085) 1007, 881 (10/16 879); at 30 Pa
-    // 689, 717, 947 (10/16 619).
-    if (h->fp64() && cfg->integrator == ICB_INTEGRATOR_BORIS && h->field_kind == kFieldUniform && !h->magnetic) {
-        double rate = 0.0;
-        for (const EnsConst& c : h->ens_const) rate = std::max(rate, c.A * c.mean_th);
-        h->spv = 16u;
-        if (rate >= 0.01) h->pend = 16u;
-    }
+    h->base_field_kind = h->field_kind;
+    default_shape(h.get(), false);
     if (cfg->pending_threshold > 0) h->pend = static_cast<uint32_t>(std::min(cfg->pending_threshold, 32));
     if (cfg->steps_per_vote > 0) h->spv = static_cast<uint32_t>(std::min(cfg->steps_per_vote, 64));
     if (cfg->stepping != ICB_STEPPING_EVENTS && cfg->stepping != ICB_STEPPING_PER_STEP &&
@@ -1305,7 +1313,6 @@ int icb_create(const icb_config* cfg, icb_handle** out) {
         ICB_CUDA(h->mix.alloc(mixes.size()));
         ICB_CUDA(cudaMemcpy(h->mix.p, mixes.data(), mixes.size() * sizeof(MixConst), cudaMemcpyHostToDevice));
     }
-    h->base_field_kind = h->field_kind;
     h->waves.assign(h->ens.size() * ICB_N_CHANNELS, icb_waveform{});
     h->wave_set.assign(h->ens.size() * ICB_N_CHANNELS, 0);
     h->tims.assign(h->ens.size(), icb_tims_field{});
