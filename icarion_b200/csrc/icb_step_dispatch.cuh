@@ -7,13 +7,21 @@
 namespace icb {
 
 // Whether the float RF / time-dependent kernel should run with room for 24
-// resident warps per SM (80 registers, some spilled) instead of 20 (96): when
-// the launch then takes enough fewer rounds of resident warps.  Every warp
+// resident warps per SM (80 registers, more of them spilled) instead of 20
+// (96): when the launch then takes fewer rounds of resident warps.  Every warp
 // runs the same number of steps, so a round that is nearly empty still costs
-// most of a round: 3,126 warps (the 100,001-ion trap on 148 SMs) are 1.06
-// rounds of 20 per SM, 0.88 of 24: 1205 -> 913 us a pass; 8,192 warps (TIMS,
-// 262,144 ions) are 3 rounds either way and slower with 24 (1679 -> 1764 us).
-inline bool more_warps(dim3 grid, dim3 block) {
+// most of a round.  Time with 24 over time with 20, trap of 22 to 72 warps of
+// ions per SM, 300 steps:
+//   2 rounds -> 1: 0.62 to 0.98 in every form (mixed and hi/lo, Boris and
+//     RK4, with and without B, collisions and a time-dependent field);
+//   3 -> 2 and 4 -> 3 (`later`): mixed Boris with collisions 0.83 to 0.98,
+//     without collisions or B 0.91 to 1.02, mixed RK4 with collisions in a
+//     constant-voltage field 0.88 to 0.99.  The others spill more than the
+//     round saves: RK4 without collisions 1.08 to 1.24, RK4 in a
+//     time-dependent field 0.98 to 1.08, no collisions with B 1.03 to 1.11,
+//     hi/lo 0.88 (network) to 1.16 (no collisions);
+//   the same number of rounds: 1.01 to 1.38.
+inline bool more_warps(dim3 grid, dim3 block, bool later) {
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1)
@@ -21,14 +29,17 @@ inline bool more_warps(dim3 grid, dim3 block) {
     const uint64_t warps = static_cast<uint64_t>(grid.x) * (block.x / 32u);
     const uint64_t a = 20ull * static_cast<uint64_t>(sms), b = 24ull * static_cast<uint64_t>(sms);
     const uint64_t ra = (warps + a - 1) / a, rb = (warps + b - 1) / b;
-    // a round of 24 warps costs about 1.26 of a round of 20
-    return 126ull * rb < 100ull * ra;
+    return rb < ra && (ra == 2u || (later && ra <= 4u));
 }
 
 template <int PREC, int INTEG, int COLL, int FIELD, bool MAG>
 cudaError_t launch_one(const StepParams& p, dim3 grid, dim3 block, cudaStream_t s) {
     if constexpr (PREC != kPrecFP64 && FIELD == kFieldLinearRF) {
-        if (p.do_push && p.do_collide && p.do_finalize && more_warps(grid, block)) {
+        constexpr bool kColl = COLL != kCollNone;
+        bool tf = false;
+        for (uint32_t e = 0; e < p.n_ens; ++e) tf = tf || p.ens[e].tf;
+        const bool later = PREC == kPrecMixed && (INTEG == kBoris ? kColl || !MAG : kColl && !tf);
+        if (p.do_push && p.do_collide && p.do_finalize && more_warps(grid, block, later)) {
             k_step<PREC, INTEG, COLL, FIELD, MAG, true, 6><<<grid, block, 0, s>>>(p);
             return cudaGetLastError();
         }
