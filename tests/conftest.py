@@ -23,6 +23,13 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA device (B200) and the built CUDA library")
 
 
+def pytest_collection_modifyitems(items):
+    """The tests that run a binary built from the reference's sources come
+    last: a run that stops at the first failure has run all others when that
+    binary could not be built."""
+    items.sort(key=lambda item: item.path.name == "test_gpu_adapters.py")
+
+
 @pytest.fixture(scope="session")
 def golden():
     def load(name: str):
