@@ -1726,8 +1726,11 @@ __global__ void __launch_bounds__(128, MIN_BLOCKS) k_step(const __grid_constant_
         // push call restarts for the collide call that follows).  An event
         // before the launch was missed (the ion was inactive at its step, the
         // engine clock was moved past it, or the caller's step left
-        // collisions out): the optical depth still left runs from here on.
-        const bool missed = static_cast<int32_t>((g_next & ~kRefresh) - step0) < 0;
+        // collisions out), and a wait that starts after this step's collide
+        // call belongs to a clock that was moved back: the optical depth
+        // still left runs from here on.
+        const bool missed = static_cast<int32_t>((g_next & ~kRefresh) - step0) < 0 ||
+                            static_cast<int32_t>(g_start - step0) > 1;
         if (live && (do_coll || do_push) && (g_next == kNeedRestart || missed)) clock_restart(step0);
     }
 

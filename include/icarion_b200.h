@@ -318,7 +318,7 @@ int icb_finalize(struct icb_handle* h, icb_run_stats* stats);
 /* Engine clock: step index and time of ensemble 0 (all ensembles share the
  * step index; time_s[e] = accumulated dt of ensemble e).  An ion whose next
  * collision event lies before the step set (as one that was inactive at that
- * step) starts a new wait there. */
+ * step), or whose wait began after it, starts a new wait there. */
 int icb_get_clock(struct icb_handle* h, uint64_t* step, double* time_s);
 int icb_set_clock(struct icb_handle* h, uint64_t step, const double* time_s);
 /* Per-ensemble moments of the active ions (ICB_N_MOMENTS doubles each). */

@@ -1287,8 +1287,10 @@ int orc_run(const orc_domain* d, int integrator, int collision, uint64_t seed,
                 sk.next = clk_next[i];
                 sk.start = clk_start[i];
                 skip_setup(&sk, d, &Gi, q, m);
-                /* also when the event lies before the call (missed) */
-                const int missed = (int32_t)((sk.next & ~ORC_REFRESH) - (uint32_t)step0) < 0;
+                /* also when the event lies before the call (missed) or the
+                 * wait starts after its first step (the clock was moved back) */
+                const int missed = (int32_t)((sk.next & ~ORC_REFRESH) - (uint32_t)step0) < 0 ||
+                                   (int32_t)(sk.start - (uint32_t)step0) > 1;
                 if (act && contains(d, p) && (sk.next == ORC_NEED_RESTART || missed)) {
                     uint64_t ov = 0;
                     skip_restart(&sk, &Gi, v, (uint32_t)step0, &ov);

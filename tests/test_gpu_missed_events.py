@@ -1,7 +1,8 @@
 """Ions whose stored clock event was not taken when its step went by: they
 were inactive then (icb_update_state, icb_advance_host), the engine clock was
 moved past it (icb_set_clock), or the caller's step left collisions out
-(push and finalize without collide).
+(push and finalize without collide).  And ions whose wait for an event began
+after the step that the engine clock was moved back to.
 
 The planned FP64 loop (launches of 8 steps or more) and the loop with
 per-step bookkeeping (up to 7) give the same bits from such a state on, the
@@ -48,7 +49,9 @@ def _ions(n=300):
 
 def _miss(sim, how, steps):
     """Lets the events of `steps` steps go by for every second ion, or for all."""
-    if how == "clock":
+    if how == "rewound":
+        sim.set_clock(0, np.zeros(1))
+    elif how == "clock":
         step, t = sim.clock()
         sim.set_clock(step + steps, t + steps * 4e-9)
     elif how == "uncollided":
@@ -75,7 +78,7 @@ def _run(per_launch, how, missed, precision=capi.PREC_FP64, collision=capi.COLLI
     with Simulation([_domain(mix)], precision=precision, collision=collision, rng_seed=5,
                     steps_per_launch=per_launch) as sim:
         sim.upload(_ions())
-        sim.advance(30)
+        sim.advance(30 if how != "rewound" else 300)
         _miss(sim, how, missed)
         rs = sim.advance(200)
         return sim.download(), rs
@@ -101,7 +104,7 @@ def test_planned_steps_equal_single_steps_after_missed_events(how, missed, colli
                                                      (capi.PREC_MIXED_HILO, capi.COLLISION_HSS, False),
                                                      (capi.PREC_MIXED, capi.COLLISION_LANGEVIN, False)])
 @pytest.mark.parametrize("per_launch", [1, 7, 1000])
-@pytest.mark.parametrize("how", ["update", "clock", "uncollided"])
+@pytest.mark.parametrize("how", ["update", "clock", "rewound", "uncollided"])
 def test_collisions_go_on_after_missed_events(how, per_launch, precision, collision, mix):
     """Counts of 200 steps after 40 missed ones against the same 200 steps
     taken at once: both Poisson-like, 5 sigma of their difference apart."""
@@ -115,13 +118,13 @@ def test_collisions_go_on_after_missed_events(how, per_launch, precision, collis
 
 @pytest.mark.parametrize("collision", [capi.COLLISION_HSS, capi.COLLISION_LANGEVIN])
 @pytest.mark.parametrize("missed", [1, 40])
-@pytest.mark.parametrize("how", ["update", "clock"])
+@pytest.mark.parametrize("how", ["update", "clock", "rewound"])
 def test_fp64_run_after_missed_events_matches_oracle(how, missed, collision):
     out, rs = _run(1000, how, missed, collision=collision)
     ens, ost = _domain(), oracle_state(_ions())
     kind = 2 if collision == capi.COLLISION_HSS else 3
-    r = orc.run(ens, ost, 30, collision=kind, seed=5)
-    step = 30 + missed
+    r = orc.run(ens, ost, 30 if how != "rewound" else 300, collision=kind, seed=5)
+    step = 30 + missed if how != "rewound" else 0
     if how == "update":
         ost["active"][::2] = 0
         r = orc.run(ens, ost, missed, collision=kind, seed=5, step0=30, t0=30 * 4e-9, clock=r["clock"])
